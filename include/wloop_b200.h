@@ -297,7 +297,9 @@ int wlg_contract_form(wlg_ctx* ctx, int* form);
  * bx an upper bound on the start slices per block, stages the copy pipeline
  * depth (2-4), cpc the column chunks per block.  Results do not depend on
  * occ, ord, bx or stages; cpc sets how the FP32 sums of the mixed form are
- * split (FP32 rounding only). */
+ * split (FP32 rounding only).  In the FP64 form any of them asks for the FMA
+ * kernel; with none, fields whose lines stay in the digits' range are
+ * multiplied as exact 8-bit digits on the tensor cores. */
 int wlg_set_gram_tuning(wlg_ctx* ctx, int occ, int ord, int bx, int stages, int cpc);
 /* The plan those settings give for msl levels and mwlt on ctx's lattice:
  * shape[10] = {extents per thread, occ, ord, start slices per block, blocks
@@ -314,6 +316,14 @@ int wlg_gram_shape(wlg_ctx* ctx, int msl, int mwlt, int* shape);
  * plan fits (the carried-line form then measures). */
 int wlg_gram_plan_shape(const int n[4], int bc, int msl, int mwlt, int precision,
                         const int tune[5], long long shape[16]);
+/* The plan of the FP64 temporal-gauge form's tensor-core Gram product for a
+ * lattice (host only): rows of the A and B digit planes, B rows per tile,
+ * 128-row A tiles, tiles, pipeline stages, TMEM columns, shared memory, column
+ * units per chunk, chunks, K blocks per work item, column splits, bytes of the
+ * A and B planes and of the sums, 32-site tiles per slice.  budget: bytes the
+ * planes may take (0: the default). */
+int wlg_slice_plan_shape(const int n[4], int bc, int msl, int mwlt, int mwlr, long long budget,
+                         long long shape[16]);
 /* The context's CUDA stream (cudaStream_t), for callers that record events. */
 void* wlg_stream(wlg_ctx* ctx);
 /* Number of wloop_b200 kernel launches issued by this process so far. */

@@ -47,12 +47,17 @@ struct Cfg {
   bool gram_ok, gram;
   GramPlan gp;
   size_t gG, gH, gUh, gB, gA, gDev;
+  // its tensor-core Gram product (gslice.cu): the digit planes take the level
+  // store, dead once the first lines exist
+  bool slices;
+  SlicePlan sp;
+  size_t gS, gAcc;
   size_t gpartial;  // byte offset of its partial sums in the partial-sum buffer
 };
 
 enum OpKind {
   OP_SMEAR, OP_COPY, OP_LINES, OP_CONTRACT, OP_REDUCE, OP_D2H,
-  OP_GRAM_CHAIN, OP_GRAM_PREP, OP_GRAM_R
+  OP_GRAM_CHAIN, OP_GRAM_PREP, OP_GRAM_R, OP_SLICES
 };
 
 struct Op {
@@ -84,7 +89,8 @@ struct wlg_batch {
   size_t pbuf_bytes = 0, pbuf_cap = 0;
   double* wl_host = nullptr;  // pinned
   size_t wl_host_doubles = 0;
-  unsigned long long* dev_host = nullptr;  // pinned: |g g^dag - 1| per lattice (bits)
+  // pinned, per lattice: |g g^dag - 1|, |U^dag U - 1| of the levels (bits), failed wait
+  unsigned long long* dev_host = nullptr;
   char* staging = nullptr;    // device AoS staging for uploads
   size_t staging_bytes = 0;
   // phase 0: smearing and the gauge chains; phase 1: the loops, per lattice
@@ -98,7 +104,9 @@ struct wlg_batch {
     cudaGraphExec_t exec = nullptr;
     int kernels = 0;  // kernels one run of the phase launches
   } ph[2];
-  std::vector<char> use_gram;  // per lattice: the temporal-gauge form runs in phase 1
+  // per lattice, phase 1: 0 carried lines, 1 temporal gauge with the FMA Gram
+  // product, 2 with the tensor-core one
+  std::vector<char> use_gram;
   bool use_graph = true;       // capture each phase after its first run and replay it
   int tG = 0, tSB = 0, tBlock = 0, tNCB = 0;  // contraction shape override (tuning)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -370,13 +378,14 @@ template <class T> void build_ops(wlg_batch* b, int phase) {
     op.cfg = c;
     sink.push_back(op);
     op.kind = OP_D2H;
-    op.dst = b->dev_host + c;
+    op.dst = b->dev_host + 3 * c;
     op.src = base(b->cfg[c].gDev);
-    op.bytes = sizeof(unsigned long long);
+    op.bytes = 2 * sizeof(unsigned long long);
     sink.push_back(op);
   }
   cur_phase = 1;
   auto gram_on = [&](int c) { return c < (int)b->use_gram.size() && b->use_gram[c]; };
+  auto slices_on = [&](int c) { return gram_on(c) && b->use_gram[c] == 2; };
 
   // ---- loops (wloop.c:524-608) ----
   // temporal-gauge lattices: the first lines, then per R their line step,
@@ -384,13 +393,13 @@ template <class T> void build_ops(wlg_batch* b, int phase) {
   for (int c = 0; c < n; c++) {
     if (!gram_on(c)) continue;
     Op op{};
-    op.kind = OP_GRAM_PREP;
+    op.kind = slices_on(c) ? OP_SLICES : OP_GRAM_PREP;
     op.cfg = c;
     sink.push_back(op);
   }
   for (int r = 0; r < maxr; r++)
     for (int c = 0; c < n; c++) {
-      if (!gram_on(c) || r >= b->cfg[c].p.mwlr) continue;
+      if (!gram_on(c) || slices_on(c) || r >= b->cfg[c].p.mwlr) continue;
       Op op{};
       op.kind = OP_GRAM_R;
       op.cfg = c;
@@ -493,6 +502,15 @@ template <class T> void build_ops(wlg_batch* b, int phase) {
     }
   }
   for (int c = 0; c < n; c++) {
+    if (!slices_on(c)) continue;
+    Op op{};
+    op.kind = OP_D2H;
+    op.dst = b->dev_host + 3 * c + 2;
+    op.src = base(b->cfg[c].gDev + 2 * sizeof(unsigned long long));
+    op.bytes = sizeof(unsigned long long);
+    sink.push_back(op);
+  }
+  for (int c = 0; c < n; c++) {
     const Cfg& f = b->cfg[c];
     Op op{};
     op.kind = OP_D2H;
@@ -515,7 +533,8 @@ template <class T> int issue(wlg_batch* b, int phase) {
     return b->side[0] ? b->side[c % wlg_batch::kSide] : b->st;
   };
   for (const Op& op : b->ph[phase].ops) {
-    const bool gram_op = op.kind == OP_GRAM_PREP || op.kind == OP_GRAM_R;
+    const bool gram_op =
+        op.kind == OP_GRAM_PREP || op.kind == OP_GRAM_R || op.kind == OP_SLICES;
     if (gram_op && !forked && b->side[0]) {
       WLG_CUDA(cudaEventRecord(b->fork, b->st));
       for (int k = 0; k < wlg_batch::kSide; k++) WLG_CUDA(cudaStreamWaitEvent(b->side[k], b->fork, 0));
@@ -562,6 +581,35 @@ template <class T> int issue(wlg_batch* b, int phase) {
                        (double*)(b->arena + f.gG), (double*)(b->arena + f.gH),
                        (unsigned long long*)(b->arena + f.gDev), b->st);
         kernels++;
+        if (f.slices) {
+          levels_deviation(f.g, f.p.msl,
+                           (const double2*)(b->arena + f.region + 6 * f.D * elem_bytes(b)),
+                           (unsigned long long*)(b->arena + f.gDev) + 1, b->st);
+          kernels++;
+        }
+        break;
+      }
+      case OP_SLICES: {
+        const Cfg& f = b->cfg[op.cfg];
+        cudaStream_t ls = lattice_stream(op.cfg);
+        double* uh = (double*)(b->arena + f.gUh);
+        double* bl = (double*)(b->arena + f.gB);
+        const double* hinv = (const double*)(b->arena + f.gH);
+        gauge_first<double>(f.g, f.gp, f.p.msl,
+                            (const double2*)(b->arena + f.region + 6 * f.D * elem_bytes(b)),
+                            (const double*)(b->arena + f.gG), hinv, uh, bl, nullptr, ls);
+        unsigned char* sa = (unsigned char*)(b->arena + f.gS);
+        unsigned char* sb = sa + align256(f.sp.bytes_a);
+        unsigned long long* acc = (unsigned long long*)(b->arena + f.gAcc);
+        int* fail = (int*)((unsigned long long*)(b->arena + f.gDev) + 2);
+        WLG_CUDA(cudaMemsetAsync(acc, 0, f.sp.acc_bytes, ls));
+        WLG_CUDA(cudaMemsetAsync(fail, 0, sizeof(unsigned long long), ls));
+        for (int ch = 0; ch < f.sp.nchunk; ch++) {
+          slice_lines(f.g, f.sp, ch, uh, bl, hinv, sa, sb, ls);
+          slice_gram(f.sp, ch, sa, sb, acc, fail, ls);
+        }
+        slice_finish(f.g, f.sp, f.bc, acc, (double*)(b->arena + f.wl), ls);
+        kernels += 2 + 2 * f.sp.nchunk;
         break;
       }
       case OP_GRAM_PREP: {
@@ -622,6 +670,7 @@ int plan(wlg_batch* b) {
     // the temporal-gauge form where it applies (phase 1 falls back to the
     // carried lines per lattice, so those get their partial sums too)
     f.gram = f.gram_ok && b->tG == 0;
+    f.slices = f.gram && f.sp.nchunk > 0;
     if (f.gram) {
       f.gpartial = poff;
       poff = align256(poff + f.gp.partial_elems * (fp64 ? 8 : 4));
@@ -676,7 +725,17 @@ void layout(wlg_batch* b) {
         o = align256(o + na);
       }
       f.gDev = f.region + o;
-      o = align256(o + 8);
+      o = align256(o + 24);
+      // digit planes in the level store; the integer sums
+      f.gS = align256(f.region + 6 * f.D * es);
+      const size_t room = f.region + lines_at - f.gS;
+      if (fp64 && room > 512 && slice_plan(f.sp, f.g, f.bc, f.p.msl, f.p.mwlt, f.p.mwlr,
+                                           std::min(room - 512, kSliceBudget))) {
+        f.gAcc = f.region + o;
+        o = align256(o + f.sp.acc_bytes);
+      } else {
+        f.sp = SlicePlan();
+      }
       if (2 * gh <= 6 * f.D * es) {
         f.gG = f.region;
         f.gH = f.region + gh;
@@ -745,7 +804,7 @@ int build(wlg_batch* b, int phase) {
   if (P.built) return 0;
   if (phase == 1)
     for (size_t c = 0; c < b->cfg.size(); c++)
-      if (c < b->use_gram.size() && b->use_gram[c] && gram_prepare(b->cfg[c].gp)) return -1;
+      if (c < b->use_gram.size() && b->use_gram[c] == 1 && gram_prepare(b->cfg[c].gp)) return -1;
   if (b->prec == WLG_FP64)
     build_ops<double>(b, phase);
   else
@@ -860,7 +919,7 @@ int wlg_batch_create(int nconf, const int* dims, const int* bcs, const wlg_wloop
   if (cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking) != cudaSuccess || ensure_pbuf(b) ||
       pool_alloc(b, &b->arena, b->arena_bytes) || pool_alloc(b, &b->staging, b->staging_bytes) ||
       cudaMallocHost(&b->wl_host, b->wl_host_doubles * sizeof(double)) != cudaSuccess ||
-      cudaMallocHost(&b->dev_host, nconf * sizeof(unsigned long long)) != cudaSuccess) {
+      cudaMallocHost(&b->dev_host, 3 * nconf * sizeof(unsigned long long)) != cudaSuccess) {
     set_error("batch_create: cannot allocate %.2f GB arena: %s", b->arena_bytes / 1e9,
               cudaGetErrorString(cudaGetLastError()));
     wlg_batch_destroy(b);
@@ -1026,9 +1085,13 @@ int wlg_batch_run(wlg_batch* b) {
   std::vector<char> use(n, 0);
   for (size_t c = 0; c < n; c++) {
     if (!b->cfg[c].gram) continue;
-    double dev;
-    memcpy(&dev, b->dev_host + c, sizeof(dev));
-    use[c] = dev <= kGramMaxDeviation;
+    double dev[2];
+    memcpy(dev, b->dev_host + 3 * c, sizeof(dev));
+    use[c] = dev[0] <= kGramMaxDeviation;
+    if (use[c] && b->cfg[c].slices && slice_in_range(dev[0], dev[1], b->cfg[c].p.mwlr) &&
+        slice_prepare() == 0)
+      use[c] = 2;
+    set_error("%s", "");
   }
   if (use != b->use_gram) {
     unbuild_phase(b, 1);
@@ -1052,6 +1115,11 @@ int wlg_batch_run(wlg_batch* b) {
     set_error("batch_run: the contraction's staged-line copies did not arrive in time");
     return -1;
   }
+  for (size_t c = 0; c < n; c++)
+    if (b->use_gram[c] == 2 && b->dev_host[3 * c + 2] != 0) {
+      set_error("batch_run: the Gram product's operand copies did not arrive in time");
+      return -1;
+    }
   // a phase that ran its ops directly is captured for the next runs
   if (b->use_graph && !captured0 && capture(b, 0)) return -1;
   if (b->use_graph && !captured1 && capture(b, 1)) return -1;

@@ -69,6 +69,8 @@ struct wlg_ctx {
   // the temporal-gauge form: g, H^-1, recursion links, B and A lines, the
   // unitarity deviation of g
   DevBuf gG, gH, gUh, gB, gA, gDev;
+  // its tensor-core Gram product: digit planes, integer sums
+  DevBuf gSa, gSb, gAcc;
   void* lines_at = nullptr;  // buffer holding the lines of length lines_len
   // after a temporal-gauge measurement the lines of length lines_lazy are
   // rebuilt from the level store when they are asked for
@@ -394,6 +396,74 @@ static void release_idle_scratch(wlg_ctx* c) {
   set_error("%s", "");
 }
 
+// The FP64 loop stage on the tensor cores (gslice.cu), once g and H^-1 exist and the
+// digits' range is known to hold: the first lines, then per chunk of columns
+// the lines of every R as digit planes and their Gram products.  Returns 1
+// (nothing done) when its buffers do not fit.
+static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan& gp,
+                           const SlicePlan& sp, double* wl_mat) {
+  const Geo& g = c->g;
+  const int msl = p->msl;
+  const size_t nb = gp.A * sizeof(double) * 3 * msl;
+  auto alloc = [&]() {
+    return ensure(c->gUh, nb) || ensure(c->gB, nb) || ensure(c->gSa, sp.bytes_a) ||
+           ensure(c->gSb, sp.bytes_b) || ensure(c->gAcc, sp.acc_bytes) ||
+           ensure(c->wl, sizeof(double) * sp.nwl);
+  };
+  if (alloc()) {
+    release_idle_scratch(c);
+    if (alloc()) {
+      set_error("%s", "");
+      release(c->gSa);
+      release(c->gSb);
+      return 1;
+    }
+  }
+  c->used_variant = 11;
+  c->lines_len = 0;
+  c->lines_at = nullptr;
+  c->lines_lazy = p->mwlr >= 2 ? p->mwlr : 0;
+  double* uh = (double*)c->gUh.p;
+  double* bl = (double*)c->gB.p;
+  const double* hinv = (const double*)c->gH.p;
+  unsigned long long* acc = (unsigned long long*)c->gAcc.p;
+  int* fail = (int*)((unsigned long long*)c->gDev.p + 2);
+  WLG_CUDA(cudaMemsetAsync(acc, 0, sp.acc_bytes, c->st));
+  WLG_CUDA(cudaMemsetAsync(fail, 0, sizeof(int), c->st));
+  {
+    ProfScope ps(c, "gauge");
+    gauge_first<double>(g, gp, msl, (const double2*)c->levels.p, (const double*)c->gG.p, hinv, uh, bl,
+                   nullptr, c->st);
+  }
+  for (int ch = 0; ch < sp.nchunk; ch++) {
+    {
+      ProfScope ps(c, "lines");
+      slice_lines(g, sp, ch, uh, bl, hinv, (unsigned char*)c->gSa.p, (unsigned char*)c->gSb.p,
+                     c->st);
+    }
+    {
+      ProfScope ps(c, "contract");
+      slice_gram(sp, ch, (unsigned char*)c->gSa.p, (unsigned char*)c->gSb.p, acc, fail, c->st);
+    }
+  }
+  {
+    ProfScope ps(c, "reduce");
+    slice_finish(g, sp, c->bc, acc, (double*)c->wl.p, c->st);
+  }
+  if (get_error()[0]) return -1;
+  int failed = 0;
+  WLG_CUDA(cudaMemcpyAsync(&failed, fail, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+  if (wl_mat)
+    WLG_CUDA(cudaMemcpyAsync(wl_mat, c->wl.p, sizeof(double) * sp.nwl, cudaMemcpyDeviceToHost,
+                             c->st));
+  WLG_CUDA(cudaStreamSynchronize(c->st));
+  if (failed) {
+    set_error("wloop_sum: the Gram product's operand copies did not arrive in time");
+    return -1;
+  }
+  return 0;
+}
+
 // wloops() in the temporal gauge (gram.cu): the gauge field and H^-1 once,
 // then the first lines; per R the line step, the banded Gram product and its
 // reduction.  Returns 1 (nothing done) when the form does not apply: shapes
@@ -405,28 +475,38 @@ static int do_loops_gram(wlg_ctx* c, const wlg_wloop_parms* p, double* wl_mat) {
   const Geo& g = c->g;
   const int msl = p->msl;
   GramPlan gp;
+  SlicePlan sp;
+  const bool fp64 = c->prec == WLG_FP64;
   // the form needs projected smearing (the projection keeps the temporal
   // links near SU(3), so g stays well conditioned)
   if (p->proj_iter < 3) return 1;
-  if (!gram_plan(gp, g, c->bc, msl, p->mwlt, c->prec == WLG_FP64, &c->gtune)) return 1;
+  const bool fma_ok = gram_plan(gp, g, c->bc, msl, p->mwlt, fp64, &c->gtune);
+  if (!fma_ok) return 1;
+  // a tuned shape asks for the FMA kernel
+  bool slices = fp64 && !c->gtune.set() && slice_plan(sp, g, c->bc, msl, p->mwlt, p->mwlr) &&
+                slice_prepare() == 0;
   if (gram_prepare(gp)) return -1;
   const size_t nb = gp.A * sizeof(T) * 3 * msl, na = gp.Aa * sizeof(T) * 3 * msl;
   const size_t nwl = (size_t)msl * msl * p->mwlt * p->mwlr * g.n[0];
   if (ensure(c->gG, gp.A * sizeof(double)) || ensure(c->gH, gp.A * sizeof(double)) ||
-      ensure(c->gDev, sizeof(unsigned long long)))
+      ensure(c->gDev, 3 * sizeof(unsigned long long)))
     return -1;
   Links<T> U = view4<T>(c->U.p, g.vol);
-  double dev = 0.0;
+  unsigned long long* devs = (unsigned long long*)c->gDev.p;  // dev, delta, failed wait
+  double dev[2] = {0.0, 0.0};
   {
     ProfScope ps(c, "gauge");
-    gauge_chain<T>(g, gp, U.p[0], (double*)c->gG.p, (double*)c->gH.p,
-                   (unsigned long long*)c->gDev.p, c->st);
-    unsigned long long bits = 0;
-    WLG_CUDA(cudaMemcpyAsync(&bits, c->gDev.p, sizeof(bits), cudaMemcpyDeviceToHost, c->st));
+    gauge_chain<T>(g, gp, U.p[0], (double*)c->gG.p, (double*)c->gH.p, devs, c->st);
+    if (slices) levels_deviation(g, msl, (const double2*)c->levels.p, devs + 1, c->st);
+    WLG_CUDA(cudaMemcpyAsync(dev, devs, sizeof(dev), cudaMemcpyDeviceToHost, c->st));
     WLG_CUDA(cudaStreamSynchronize(c->st));
-    memcpy(&dev, &bits, sizeof(dev));
   }
-  if (!(dev <= kGramMaxDeviation)) return 1;
+  if (!(dev[0] <= kGramMaxDeviation)) return 1;
+  slices = slices && slice_in_range(dev[0], dev[1], p->mwlr);
+  if (slices) {
+    const int rc = do_loops_slices(c, p, gp, sp, wl_mat);
+    if (rc != 1) return rc;
+  }
   auto alloc = [&]() {
     return ensure(c->gUh, nb) || ensure(c->gB, nb) || ensure(c->gA, na) ||
            ensure(c->partial, gp.partial_elems * sizeof(T)) || ensure(c->wl, sizeof(double) * nwl);
@@ -660,6 +740,9 @@ int wlg_free_scratch(wlg_ctx* c) {
   release(c->gB);
   release(c->gA);
   release(c->gDev);
+  release(c->gSa);
+  release(c->gSb);
+  release(c->gAcc);
   c->lines_at = nullptr;
   c->lines_len = 0;
   c->lines_lazy = 0;
@@ -675,7 +758,7 @@ int wlg_destroy(wlg_ctx* c) {
   if (c->cst) cudaStreamSynchronize(c->cst);
   harvest(c);
   DevBuf* all[] = {&c->U, &c->U0, &c->bar, &c->til, &c->apeA, &c->apeB, &c->dl, &c->levels, &c->lines, &c->lines2,
-                   &c->gG, &c->gH, &c->gUh, &c->gB, &c->gA, &c->gDev, &c->partial, &c->wl, &c->plaq_part, &c->plaq_out, &c->staging, &c->ipt,
+                   &c->gG, &c->gH, &c->gUh, &c->gB, &c->gA, &c->gDev, &c->gSa, &c->gSb, &c->gAcc, &c->partial, &c->wl, &c->plaq_part, &c->plaq_out, &c->staging, &c->ipt,
                    &c->prefetch_buf};
   for (DevBuf* b : all) release(*b);
   for (cudaEvent_t e : c->evpool) cudaEventDestroy(e);
@@ -1229,6 +1312,35 @@ int wlg_gram_plan_shape(const int n[4], int bc, int msl, int mwlt, int precision
   const long long v[16] = {gp.TQ, gp.occ, gp.ord + 1, gp.BX, gp.BXp, gp.NG, gp.NYB, gp.NYBp,
                            gp.nblk, gp.nrows, gp.stages, gp.block, (long long)gp.smem,
                            gp.nchunks, gp.cpc, gp.nsplit};
+  for (int i = 0; i < 16; i++) shape[i] = v[i];
+  return 0;
+}
+
+int wlg_slice_plan_shape(const int n[4], int bc, int msl, int mwlt, int mwlr, long long budget,
+                         long long shape[16]) {
+  set_error("%s", "");
+  if (!n || !shape || (bc != 0 && bc != 3) || budget < 0) {
+    set_error("slice_plan_shape: bad arguments");
+    return -1;
+  }
+  for (int i = 0; i < 4; i++)
+    if (n[i] < 2) {
+      set_error("slice_plan_shape: lattice extent N%d=%d < 2", i, n[i]);
+      return -1;
+    }
+  if ((long long)n[0] * n[1] * n[2] * n[3] > (1LL << 30)) {
+    set_error("slice_plan_shape: lattice volume too large");
+    return -1;
+  }
+  SlicePlan sp;
+  if (!slice_plan(sp, make_geo(n), bc, msl, mwlt, mwlr, budget ? (size_t)budget : kSliceBudget)) {
+    set_error("no digit-plane plan for msl %d, mwlt %d, mwlr %d", msl, mwlt, mwlr);
+    return -1;
+  }
+  const long long v[16] = {sp.rows_a, sp.rows_b, sp.TN, sp.nmt, sp.ntiles, sp.stages,
+                           sp.tmem_cols, (long long)sp.smem, sp.nuc, sp.nchunk, sp.kps, sp.nsplit,
+                           (long long)sp.bytes_a, (long long)sp.bytes_b, (long long)sp.acc_bytes,
+                           sp.ntile};
   for (int i = 0; i < 16; i++) shape[i] = v[i];
   return 0;
 }

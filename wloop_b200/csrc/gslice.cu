@@ -1,0 +1,774 @@
+// gslice.cu -- the FP64 form's temporal-gauge loop stage (gram.cu's identities
+// and slab layout) with the banded Gram product on the tensor cores, exactly:
+// the lines are written as signed 8-bit digits and multiplied by tcgen05.mma
+// of kind::i8 with 32-bit integer accumulation.
+//
+//     x = sum_p q_p 2^(-6-8p),  q_p in [-128, 127],  p < 7
+//
+// (x rounded to 2^-54; |x| < 1.99).  A line entry is bounded by the product of
+// the operator norms it is made of, so the host admits a lattice only if
+//     (1 + 3 delta)^(R/2) / (1 - 3 dev) <= 1.98
+// (delta, dev: largest |U^dag U - 1| over the stored levels and |g g^dag - 1|
+// over the gauge field); the FMA kernel of gram.cu measures the others, and
+// a NaN anywhere fails the comparison.  A dot product is then
+//     sum_c a_c b_c = sum_m 2^(-12-8m) C_m,   C_m = sum_{i+j=m} q_a,i . q_b,j
+// over the classes m < 7.  The classes that are left out and the rounding of x
+// are unbiased digits of size 2^-54 per column, and shrink against the sum
+// with the square root of the 54 N1 N2 N3 columns, to below 1e-17 of W; the
+// integer sums are exact, so a result does not depend on how columns are split
+// over blocks or in which order blocks add theirs.  Against 64-bit loops of
+// the same fields W is 1.3e-16 .. 4.9e-16 off (2-norm) where the FMA kernel's
+// FP64 sums are 4.1e-16 .. 6.5e-16 off.
+//
+// The mixed form keeps FP32 FMAs in gram.cu: its sums' rounding is part of its
+// results.
+//
+// Work is cut into chunks of column units (a unit: one direction, one 32-site
+// tile).  Per chunk k_slice_lines walks the lines of its units through all
+// spatial extents R = 1..mwlr in registers and writes the digit planes of
+// every R; k_slice_gram then forms all R's sums of the chunk.  The first
+// lines and the recursion links are read from HBM once per measurement
+// (per R before), and the chunk bounds the memory the planes take.
+//
+// Plane layout, one buffer for the A rows (start slice, level) and one for the
+// B rows (unrolled slice, level), row = slice * L + level: per (R, unit, row)
+// the P x 576 digits of one 32-site tile as 9 K blocks of 64 columns,
+//     byte (((r * nuc + unit) * rows + row) * 9 + b) * P * 64 + p * 64 + i
+// where block b < 8 holds the first 16 components of lanes 4 b .. 4 b + 3 and
+// block 8 the last two components of all lanes (the columns of a sum may come
+// in any order): a lane writes 16 bytes and 2 bytes per plane at offsets the
+// compiler knows, a warp one contiguous row, and an operand tile (rows x
+// planes of one K block) is one TMA box.
+#include <cuda.h>
+
+#include <algorithm>
+#include <cmath>
+#include <mutex>
+#include <set>
+#include <utility>
+
+#include "internal.h"
+#include "mbar.cuh"
+#include "slab.cuh"
+
+namespace wlg {
+namespace {
+
+constexpr int kPlanes = 7;
+constexpr int kKB = 64;       // bytes (columns) per K block: 32 sites x {re, im} of one entry
+constexpr int kMaxStages = 8;
+constexpr int kGramThreads = 192;  // producer warp, MMA warp, four epilogue warps
+
+// ---------------------------------------------------------------------------
+// digits
+// ---------------------------------------------------------------------------
+// Two roundings by magic addition: t1 = x + 1.5 2^22 rounds x to 2^-30, its low
+// word is round(x 2^30); the remainder (exact, at most 2^-31) plus 0.375 rounds
+// to 2^-54.  The low part may round up to 2^23, its carry goes into the high
+// part.  Bytes below the top one carry a bias of 128, taken off by the flip of
+// their top bit.
+struct Digits {
+  struct Raw {
+    unsigned ha, hb, la, lb;
+  };
+  __device__ static __forceinline__ void bits(unsigned& hi, unsigned& lo, double x) {
+    constexpr double M1 = 6291456.0;  // 1.5 * 2^22: unit in the last place 2^-30
+    const double t1 = x + M1;
+    const double m = x - (t1 - M1);
+    const double t2 = m + 0.375;      // unit in the last place 2^-54
+    lo = (unsigned)__double2loint(t2) + 0x00808080u;
+    hi = (unsigned)__double2loint(t1) + ((int)lo >> 24) + 0x00808080u;
+  }
+  __device__ static __forceinline__ Raw raw(double2 v) {
+    Raw x;
+    bits(x.ha, x.la, v.x);
+    bits(x.hb, x.lb, v.y);
+    return x;
+  }
+  __device__ static __forceinline__ void half(unsigned (&w)[kPlanes], const Raw& x) {
+    w[0] = __byte_perm(x.ha, x.hb, 0x0073);
+    w[1] = __byte_perm(x.ha, x.hb, 0x0062);
+    w[2] = __byte_perm(x.ha, x.hb, 0x0051);
+    w[3] = __byte_perm(x.ha, x.hb, 0x0040);
+    w[4] = __byte_perm(x.la, x.lb, 0x0062);
+    w[5] = __byte_perm(x.la, x.lb, 0x0051);
+    w[6] = __byte_perm(x.la, x.lb, 0x0040);
+  }
+  static constexpr unsigned flip(int p) { return p == 0 ? 0u : 0x80808080u; }
+};
+
+// the digit planes of one matrix into its row (this lane's 16 + 2 bytes per
+// plane); lanes without a site write zeros
+__device__ __forceinline__ void store_digits(unsigned char* __restrict__ o16,
+                                             unsigned char* __restrict__ o2, const M3<double>& m,
+                                             bool live) {
+  constexpr int P = kPlanes;
+  uint4 q[P];
+#pragma unroll
+  for (int h = 0; h < 4; h++) {
+    unsigned w0[P], w1[P];
+    Digits::half(w0, Digits::raw(m.e[2 * h]));
+    Digits::half(w1, Digits::raw(m.e[2 * h + 1]));
+#pragma unroll
+    for (int p = 0; p < P; p++) {
+      unsigned v = __byte_perm(w0[p], w1[p], 0x5410);
+      if (Digits::flip(p)) v ^= Digits::flip(p);
+      v = live ? v : 0u;
+      if (h == 0) q[p].x = v;
+      if (h == 1) q[p].y = v;
+      if (h == 2) q[p].z = v;
+      if (h == 3) q[p].w = v;
+    }
+  }
+  unsigned w[P];
+  Digits::half(w, Digits::raw(m.e[8]));
+#pragma unroll
+  for (int p = 0; p < P; p++) {
+    *reinterpret_cast<uint4*>(o16 + p * kKB) = q[p];
+    const unsigned v = w[p] ^ (Digits::flip(p) & 0xffffu);
+    *reinterpret_cast<unsigned short*>(o2 + p * kKB) = (unsigned short)(live ? v : 0u);
+  }
+}
+
+// tile of unit index v (0 <= v < ntile) for direction k: for k = 0 the tiles
+// along the x1 line are consecutive, so that the shifted links a chunk reads
+// are those of its own units (k = 1, 2: the lexicographic order has that)
+__device__ __forceinline__ int unit_tile(const Geo& g, int ntile, int k, int v) {
+  if (k != 0) return v;
+  const int tp = max(1, min(ntile, (g.st[1] + 16) >> 5));  // tiles per x1 plane, rounded
+  const int q = ntile / tp, rem = ntile - q * tp;
+  // column m holds tiles m, m + tp, ...: q + 1 of them for m < rem, else q
+  if (v < rem * (q + 1)) return v / (q + 1) + (v % (q + 1)) * tp;
+  const int w = v - rem * (q + 1);
+  return rem + w / q + (w % q) * tp;
+}
+
+struct LineArgs {
+  Geo g;
+  int Nu, ntile, msl, mwlr, u0, cur, nuc;
+  size_t A;  // elements of one slab array
+  const double *uh, *bl, *hinv;
+  unsigned char *sa, *sb;
+};
+
+// B(x, R) and A(x, R) = H^-1(x) B(x, R) H^-1(x + R k) for R = 1..mwlr, as
+// digit planes.  One warp per (y0, unit, level), levels in neighbouring warps
+// (they share the H^-1 tiles), the walk over R in registers.
+__global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
+  constexpr int P = kPlanes;
+  constexpr int PITCH = 9 * P * kKB;  // bytes of one row
+  const int lane = threadIdx.x & 31;
+  unsigned w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lev = (int)(w % a.msl);
+  w /= a.msl;
+  const int ul = (int)(w % a.cur);
+  const int y0 = (int)(w / a.cur);
+  if (y0 >= a.Nu) return;
+  const Geo& g = a.g;
+  const int u = a.u0 + ul, k = u / a.ntile;
+  const int jt = unit_tile(g, a.ntile, k, u - k * a.ntile);
+  const bool live = jt * 32 + lane < g.vs;
+  const int j = live ? jt * 32 + lane : g.vs - 1;
+  const bool start = y0 < g.n[0];
+  // slices of this y0: the recursion links of (level, k), and H^-1
+  const size_t slice = (size_t)y0 * a.ntile * kSlabTile;
+  const double* uh = a.uh + (size_t)(lev * 3 + k) * a.A + slice;
+  const double* hinv = a.hinv + slice;
+  const int nk = k == 0 ? g.n[1] : (k == 1 ? g.n[2] : g.n[3]);
+  const int st = k == 0 ? g.st[1] : (k == 1 ? g.st[2] : 1);
+  int z = j, y = (j / st) % nk;  // x + (R - 1) k and its coordinate along k
+  const size_t rows_a = (size_t)g.n[0] * a.msl, rows_b = (size_t)a.Nu * a.msl;
+  const int row = y0 * a.msl + lev;
+  const unsigned at16 = (unsigned)((lane >> 2) * P * kKB + (lane & 3) * 16);
+  const unsigned at2 = (unsigned)(8 * P * kKB + lane * 2);
+  unsigned char* ob = a.sb + (ul * rows_b + row) * PITCH;
+  unsigned char* oa = a.sa + (ul * rows_a + row) * PITCH;
+  const size_t step_b = a.nuc * rows_b * PITCH, step_a = a.nuc * rows_a * PITCH;
+  M3<double> c, f, t;
+  ld_slab_as(c, a.bl + (size_t)(lev * 3 + k) * a.A + slice, j >> 5, j & 31);
+#pragma unroll 1
+  for (int R = 1; R <= a.mwlr; R++) {
+    if (R > 1) {
+      ld_slab_as(f, uh, z >> 5, z & 31);
+      mul(t, c, f);
+      c = t;
+    }
+    z += st;
+    if (++y == nk) {
+      y = 0;
+      z -= nk * st;
+    }
+    store_digits(ob + at16, ob + at2, c, live);
+    if (start) {
+      ld_slab_as(f, hinv, z >> 5, z & 31);
+      mul(t, c, f);
+      ld_slab_as(f, hinv, j >> 5, j & 31);
+      M3<double> s;
+      mul(s, f, t);
+      store_digits(oa + at16, oa + at2, s, live);
+    }
+    ob += step_b;
+    oa += step_a;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The banded Gram product of one chunk.  A work item is (R, column split,
+// tile); a tile is 128 A rows against TN of the B rows their band reaches.
+// One CTA per SM walks items; per 64-column block the producer thread fetches
+// the P x 128 and P x TN digit rows with two TMA boxes (64-byte swizzle), the
+// MMA thread issues the digit pairs i + j < P, the pairs of one A plane with
+// neighbouring B planes as one MMA of up to 256 columns (their accumulators,
+// the classes i + j, are neighbours in TMEM too), and the epilogue warps read
+// the classes, combine them as 64-bit integers and add the entries inside the
+// band to the result with integer atomics.  Every wait is bounded: one that
+// runs out sets *fail, and all roles leave.
+// ---------------------------------------------------------------------------
+struct GramTileArgs {
+  int N0, Nu, L, mwlt, mwlr;
+  int rows_a, rows_b, TN, nmt, ntiles;
+  int kstride;  // K blocks of one R in the plane buffers
+  int kcur;     // K blocks of one R in this chunk
+  int kps, nsplit, stages;
+  unsigned tmem_cols;
+  long long nwl;
+  unsigned long long* acc;  // [2][nwl]: 2^24 times the first plus the second
+  int* fail;
+};
+
+struct TileAt {
+  int r, kb0, nkb, m0, b0;
+};
+
+// B rows a 128-row A tile reaches: [first, last)
+__host__ __device__ __forceinline__ void band_rows(int L, int mwlt, int rows_a, int rows_b, int m0,
+                                                   int& first, int& last) {
+  const int m1 = m0 + 127 < rows_a ? m0 + 127 : rows_a - 1;
+  first = (m0 / L + 1) * L;
+  last = (m1 / L + mwlt + 1) * L;
+  if (last > rows_b) last = rows_b;
+  if (first > last) first = last;
+}
+
+__device__ __forceinline__ TileAt tile_at(const GramTileArgs& a, long long it) {
+  TileAt t;
+  int tile = (int)(it % a.ntiles);
+  it /= a.ntiles;
+  const int sp = (int)(it % a.nsplit);
+  t.r = (int)(it / a.nsplit);
+  t.kb0 = t.r * a.kstride + sp * a.kps;
+  t.nkb = min(a.kps, a.kcur - sp * a.kps);
+  t.m0 = t.b0 = 0;
+  for (int m = 0; m < a.nmt; m++) {
+    int first, last;
+    band_rows(a.L, a.mwlt, a.rows_a, a.rows_b, m * 128, first, last);
+    const int n = (last - first + a.TN - 1) / a.TN;
+    if (tile < n) {
+      t.m0 = m * 128;
+      t.b0 = first + tile * a.TN;
+      break;
+    }
+    tile -= n;
+  }
+  return t;
+}
+
+__device__ __forceinline__ void tma_box(unsigned dst, const CUtensorMap* map, int row, int b, int u,
+                                        uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3, %2, %4, %5}], [%6];\n" ::"r"(dst),
+      "l"(map), "r"(0), "r"(row), "r"(b), "r"(u), "r"(smem_addr(bar))
+      : "memory");
+}
+
+// K-major shared-memory operand with 64-byte swizzle: 8-row groups of 512 bytes
+__device__ __forceinline__ uint64_t operand_desc(unsigned addr) {
+  return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)1 << 16) | ((uint64_t)(512 >> 4) << 32) |
+         ((uint64_t)1 << 46) | ((uint64_t)4 << 61);
+}
+
+__device__ __forceinline__ void mma_i8(unsigned d, uint64_t da, uint64_t db, unsigned idesc,
+                                       bool accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      "l"(da), "l"(db), "r"(idesc), "r"((unsigned)accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                   smem_addr(bar))
+               : "memory");
+}
+__device__ __forceinline__ void tc_fence_after() {
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+}
+__device__ __forceinline__ void tc_fence_before() {
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_addr(bar)) : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(int (&v)[16], unsigned addr) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+        "=r"(v[14]), "=r"(v[15])
+      : "r"(addr));
+}
+__device__ __forceinline__ void tmem_ld_wait() {
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+
+// bounded wait that also ends when another role has given up
+__device__ __forceinline__ bool wait_or_quit(uint64_t* bar, unsigned phase, volatile int* quit) {
+  if (mbar_try_wait(bar, phase)) return true;
+  const uint64_t t0 = global_ns();
+  while (!mbar_try_wait(bar, phase)) {
+    if (*quit) return false;
+    if (global_ns() - t0 > 2000000000ull) {
+      *quit = 1;
+      return false;
+    }
+  }
+  return true;
+}
+
+__global__ void __launch_bounds__(kGramThreads, 1)
+    k_slice_gram(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                 const GramTileArgs a) {
+  constexpr int P = kPlanes;
+  extern __shared__ unsigned char raw[];
+  __shared__ __align__(8) uint64_t full[kMaxStages], empty[kMaxStages], acc_full, acc_empty, drain;
+  __shared__ unsigned tmem_base;
+  __shared__ int quit;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned base = (smem_addr(raw) + 1023u) & ~1023u;
+  const unsigned bytes_a = P * 128 * kKB, bytes_b = (unsigned)(P * a.TN * kKB);
+  const unsigned stage_bytes = bytes_a + bytes_b;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < a.stages; s++) {
+      mbar_init(full + s, 1);
+      mbar_init(empty + s, 1);
+    }
+    mbar_init(&acc_full, 1);
+    mbar_init(&acc_empty, 4);
+    mbar_init(&drain, 1);
+    mbar_init_fence();
+    quit = 0;
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
+                     smem_addr(&tmem_base)),
+                 "r"(a.tmem_cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const unsigned tmem = tmem_base;
+  const long long items = (long long)a.mwlr * a.nsplit * a.ntiles;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int s = 0;
+      unsigned ph = 0;
+      long long issued = 0;
+      bool ok = true;
+      for (long long it = blockIdx.x; ok && it < items; it += gridDim.x) {
+        const TileAt t = tile_at(a, it);
+        for (int kb = 0; kb < t.nkb; kb++) {
+          if (!wait_or_quit(empty + s, ph ^ 1, &quit)) {
+            ok = false;
+            break;
+          }
+          const unsigned dst = base + s * stage_bytes;
+          mbar_expect_tx(full + s, stage_bytes);
+          const int un = (t.kb0 + kb) / 9, bl = t.kb0 + kb - un * 9;
+          tma_box(dst, &map_a, t.m0, bl, un, full + s);
+          tma_box(dst + bytes_a, &map_b, t.b0, bl, un, full + s);
+          issued++;
+          if (++s == a.stages) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+      }
+      if (!ok) {
+        // the copies in flight, the last use of each stage
+        for (long long b = issued > a.stages ? issued - a.stages : 0; b < issued; b++)
+          mbar_wait_bounded(full + b % a.stages, (unsigned)((b / a.stages) & 1));
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int s = 0;
+      unsigned ph = 0, aph = 0;
+      bool ok = true;
+      const int gp = 256 / a.TN;  // B planes one MMA covers
+      const unsigned idesc0 = (2u << 4) | (1u << 7) | (1u << 10) | (8u << 24);  // S32, S8 x S8, M 128
+      for (long long it = blockIdx.x; ok && it < items; it += gridDim.x) {
+        const TileAt t = tile_at(a, it);
+        if (t.nkb <= 0) continue;
+        if (!(ok = wait_or_quit(&acc_empty, aph ^ 1, &quit))) break;
+        tc_fence_after();
+        for (int kb = 0; kb < t.nkb; kb++) {
+          if (!(ok = wait_or_quit(full + s, ph, &quit))) break;
+          tc_fence_after();
+          const unsigned sa = base + s * stage_bytes, sb = sa + bytes_a;
+#pragma unroll
+          for (int ks = 0; ks < kKB / 32; ks++)
+#pragma unroll
+            for (int i = 0; i < P; i++) {
+              const uint64_t da = operand_desc(sa + i * 128 * kKB + ks * 32);
+              for (int jp = 0; jp < P - i; jp += gp) {
+                const int n = min(gp, P - i - jp) * a.TN;
+                mma_i8(tmem + (unsigned)((i + jp) * a.TN), da,
+                       operand_desc(sb + (unsigned)(jp * a.TN) * kKB + ks * 32),
+                       idesc0 | ((unsigned)(n >> 3) << 17), kb > 0 || ks > 0 || i > 0);
+              }
+            }
+          mma_commit(empty + s);
+          if (++s == a.stages) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+        if (!ok) break;
+        mma_commit(&acc_full);
+        aph ^= 1;
+      }
+      if (!ok) {  // the MMAs in flight
+        mma_commit(&drain);
+        mbar_wait_bounded(&drain, 0);
+      }
+    }
+  } else {
+    const int quad = warp & 3;
+    unsigned ph = 0;
+    for (long long it = blockIdx.x; it < items; it += gridDim.x) {
+      const TileAt t = tile_at(a, it);
+      if (t.nkb <= 0) continue;
+      if (!__all_sync(0xffffffffu, wait_or_quit(&acc_full, ph, &quit))) break;
+      tc_fence_after();
+      ph ^= 1;
+      const int r0 = t.m0 + quad * 32;
+      if (r0 < a.rows_a) {
+        const int row = r0 + lane, x0 = row / a.L, s1 = row - x0 * a.L;
+        // the columns any row of this warp needs
+        const int lo = max(0, (r0 / a.L + 1) * a.L - t.b0);
+        const int hi = min(min(a.TN, a.rows_b - t.b0),
+                           (min(r0 + 31, a.rows_a - 1) / a.L + a.mwlt + 1) * a.L - t.b0);
+        const bool live = row < a.rows_a;
+        for (int c0 = lo & ~15; c0 < hi; c0 += 16) {
+          int v[P][16];
+#pragma unroll
+          for (int m = 0; m < P; m++)
+            tmem_ld16(v[m], tmem + ((unsigned)(quad * 32) << 16) + (unsigned)(m * a.TN + c0));
+          tmem_ld_wait();
+          int e = (t.b0 + c0) / a.L, s2 = t.b0 + c0 - e * a.L;
+#pragma unroll
+          for (int c = 0; c < 16; c++) {
+            const int T = e - x0;
+            if (live && c0 + c < hi && T >= 1 && T <= a.mwlt) {
+              const long long o =
+                  s1 + (long long)a.L * (s2 + (long long)a.L *
+                                                  ((T - 1) + (long long)a.mwlt *
+                                                                 (t.r + (long long)a.mwlr * x0)));
+              const long long zh = ((long long)v[0][c] << 24) + ((long long)v[1][c] << 16) +
+                                   ((long long)v[2][c] << 8) + v[3][c];
+              const long long zl = ((long long)v[4][c] << 16) + ((long long)v[5][c] << 8) + v[6][c];
+              atomicAdd(a.acc + o, (unsigned long long)zh);
+              atomicAdd(a.acc + a.nwl + o, (unsigned long long)zl);
+            }
+            if (++s2 == a.L) {
+              s2 = 0;
+              e++;
+            }
+          }
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && quit) atomicExch(a.fail, 1);
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem),
+                 "r"(a.tmem_cols));
+}
+
+// wl = the integer sums scaled; loops through the last slice of open time are
+// exact zeros
+__global__ void __launch_bounds__(256) k_slice_finish(const long long* __restrict__ acc,
+                                                      long long nwl, int N0, int mwlt, int mwlr,
+                                                      int LL, int open, double norm,
+                                                      double* __restrict__ wl) {
+  for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < nwl;
+       o += (long long)gridDim.x * blockDim.x) {
+    const int t = (int)((o / LL) % mwlt), x0 = (int)(o / ((long long)LL * mwlt * mwlr));
+    double v = 0.0;
+    if (!open || x0 + t + 1 < N0) {
+      v = fma((double)acc[o], 0x1p-36, (double)acc[nwl + o] * 0x1p-60) / norm;
+    }
+    wl[o] = v;
+  }
+}
+
+// max |U^dag U - 1| over the stored levels, as the bits of a non-negative
+// double (a NaN counts as the largest value)
+__global__ void __launch_bounds__(256) k_levels_dev(const double2* __restrict__ lev,
+                                                    size_t stride, int narr, int vol,
+                                                    unsigned long long* __restrict__ dev) {
+  double worst = 0.0;
+  const long long n = (long long)narr * vol;
+  for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < n;
+       w += (long long)gridDim.x * blockDim.x) {
+    const int q = (int)(w / vol), s = (int)(w - (long long)q * vol);
+    M3<double> u;
+    ld<double>(u, lev + q * stride, vol, s);
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+#pragma unroll
+      for (int j = i; j < 3; j++) {
+        double re = i == j ? -1.0 : 0.0, im = 0.0;
+#pragma unroll
+        for (int m = 0; m < 3; m++) {
+          const double2 a = u.e[3 * m + i], b = u.e[3 * m + j];
+          re = fma(a.x, b.x, fma(a.y, b.y, re));
+          im = fma(a.x, b.y, fma(-a.y, b.x, im));
+        }
+        re = fabs(re);
+        im = fabs(im);
+        if (!(re <= worst)) worst = re;
+        if (!(im <= worst)) worst = im;
+      }
+  }
+  double d = worst != worst ? 1e300 : worst;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) d = fmax(d, __shfl_xor_sync(0xffffffffu, d, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(dev, (unsigned long long)__double_as_longlong(d));
+}
+
+constexpr size_t kSmemMax = 227 * 1024 - 1024;  // beside the barriers and the alignment slack
+// K blocks one 32-bit accumulation takes: the last class adds P products of
+// at most 2^14 a column, 64 columns a block
+constexpr int kRunMax = (int)((1ll << 31) / ((long long)kPlanes * (1 << 14) * kKB)) - 1;
+
+typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                             const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                             CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
+                             CUtensorMapFloatOOBfill);
+
+EncodeFn encode_fn() {
+  static EncodeFn fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult res;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault,
+                                         &res) != cudaSuccess ||
+        res != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+    return (EncodeFn)p;
+  }();
+  return fn;
+}
+
+// planes as a tensor of (64 bytes, rows, planes, blocks, (R, unit)); box: `box`
+// rows of all planes of one K block
+bool plane_map(CUtensorMap* m, void* base, int rows, long long units, int box) {
+  constexpr int P = kPlanes;
+  EncodeFn fn = encode_fn();
+  if (!fn) return false;
+  const cuuint64_t pitch = (cuuint64_t)9 * P * kKB;
+  const cuuint64_t dim[5] = {kKB, (cuuint64_t)rows, (cuuint64_t)P, 9, (cuuint64_t)units};
+  const cuuint64_t str[4] = {pitch, kKB, (cuuint64_t)P * kKB, pitch * rows};
+  const cuuint32_t bx[5] = {kKB, (cuuint32_t)box, (cuuint32_t)P, 1, 1}, one[5] = {1, 1, 1, 1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, base, dim, str, bx, one,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+}  // namespace
+
+bool slice_plan(SlicePlan& p, const Geo& g, int bc, int msl, int mwlt, int mwlr,
+                size_t budget) {
+  p = SlicePlan();
+  if (msl < 1 || msl > 8 || mwlt < 1 || mwlr < 1) return false;
+  p.L = msl;
+  p.N0 = g.n[0];
+  p.Nu = g.n[0] + (bc == 0 ? 0 : mwlt);
+  p.mwlt = mwlt;
+  p.mwlr = mwlr;
+  p.ntile = (g.vs + 31) / 32;
+  p.rows_a = p.N0 * msl;
+  p.rows_b = p.Nu * msl;
+  p.nmt = (p.rows_a + 127) / 128;
+  // B rows per tile: the band of a 128-row tile in the fewest equal tiles
+  // whose P classes fit the 512 TMEM columns
+  constexpr int nmax = (512 / kPlanes) & ~15;
+  int widest = 0;
+  for (int m = 0; m < p.nmt; m++) {
+    int first, last;
+    band_rows(msl, mwlt, p.rows_a, p.rows_b, m * 128, first, last);
+    widest = std::max(widest, last - first);
+  }
+  if (widest == 0) return false;
+  const int parts = (widest + nmax - 1) / nmax;
+  p.TN = (((widest + parts - 1) / parts) + 15) & ~15;
+  for (int m = 0; m < p.nmt; m++) {
+    int first, last;
+    band_rows(msl, mwlt, p.rows_a, p.rows_b, m * 128, first, last);
+    p.ntiles += (last - first + p.TN - 1) / p.TN;
+  }
+  const size_t stage = (size_t)kPlanes * kKB * (128 + p.TN);
+  p.stages = (int)std::min<size_t>(kMaxStages, (kSmemMax - 1024) / stage);
+  if (p.stages < 2) return false;
+  // more than half of an SM's shared memory: one CTA, one TMEM owner per SM
+  p.smem = std::max<size_t>(p.stages * stage + 1024, 116 * 1024);
+  p.tmem_cols = 32;
+  while (p.tmem_cols < kPlanes * p.TN) p.tmem_cols *= 2;
+  // column units per chunk: as many as the budget holds, in equal chunks
+  const int units = 3 * p.ntile;
+  const size_t unit = (size_t)mwlr * 9 * kPlanes * kKB * (p.rows_a + p.rows_b);
+  long long nuc = (long long)(budget / unit);
+  if (nuc < 1) return false;
+  if (nuc > units) nuc = units;
+  p.nchunk = (int)((units + nuc - 1) / nuc);
+  p.nuc = (units + p.nchunk - 1) / p.nchunk;
+  p.nchunk = (units + p.nuc - 1) / p.nuc;
+  const size_t kb = (size_t)mwlr * p.nuc * 9;
+  p.bytes_a = kb * kPlanes * p.rows_a * kKB;
+  p.bytes_b = kb * kPlanes * p.rows_b * kKB;
+  p.nwl = (size_t)msl * msl * mwlt * mwlr * p.N0;
+  p.acc_bytes = p.nwl * 2 * sizeof(unsigned long long);
+  // column splits: enough for the 32-bit range, then the fewest waves of the
+  // SMs, an item costing its K blocks and about 6 more for its epilogue
+  const int kc = p.nuc * 9, lo = (kc + kRunMax - 1) / kRunMax;
+  const long long per = (long long)mwlr * p.ntiles;
+  double best = 1e300;
+  for (int ns = lo; ns <= std::min(kc, std::max(lo, lo * 16 + 160)); ns++) {
+    const int kps = (kc + ns - 1) / ns;
+    const long long items = per * ((kc + kps - 1) / kps);
+    const double cost = (double)((items + num_sms() - 1) / num_sms()) * (kps + 6);
+    if (cost < best * 0.999) {
+      best = cost;
+      p.kps = kps;
+      p.nsplit = (kc + kps - 1) / kps;
+    }
+  }
+  return true;
+}
+
+bool slice_in_range(double dev, double delta, int mwlr) {
+  if (!(dev < 0.3) || !(delta < 0.3)) return false;
+  return std::pow(1.0 + 3.0 * delta, 0.5 * mwlr) / (1.0 - 3.0 * dev) <= 1.98;
+}
+
+int slice_prepare() {
+  void* fn = (void*)k_slice_gram;
+  static std::mutex mu;
+  static std::set<std::pair<int, void*>> done;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  if (done.count({dev, fn})) return 0;
+  if (!encode_fn()) {
+    set_error("slice gram: the driver has no cuTensorMapEncodeTiled");
+    return -1;
+  }
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax) !=
+      cudaSuccess) {
+    set_error("slice gram: %zu bytes of shared memory per block: %s", kSmemMax,
+              cudaGetErrorString(cudaGetLastError()));
+    return -1;
+  }
+  done.insert({dev, fn});
+  return 0;
+}
+
+void levels_deviation(const Geo& g, int msl, const double2* levels,
+                      unsigned long long* dev, cudaStream_t st) {
+  cudaMemsetAsync(dev, 0, sizeof(unsigned long long), st);
+  const long long n = (long long)3 * msl * g.vol;
+  const long long grid = std::min<long long>((n + 255) / 256, num_sms() * 16);
+  k_levels_dev<<<(int)grid, 256, 0, st>>>(levels, link_elems<double>(g.vol), 3 * msl, g.vol, dev);
+  WLG_LAUNCH_CHECK("levels_dev");
+}
+
+void slice_lines(const Geo& g, const SlicePlan& p, int chunk, const double* uh,
+                 const double* blines, const double* hinv, unsigned char* sa, unsigned char* sb, cudaStream_t st) {
+  LineArgs a;
+  a.g = g;
+  a.Nu = p.Nu;
+  a.ntile = p.ntile;
+  a.msl = p.L;
+  a.mwlr = p.mwlr;
+  a.u0 = chunk * p.nuc;
+  a.cur = std::min(p.nuc, 3 * p.ntile - a.u0);
+  a.nuc = p.nuc;
+  a.A = (size_t)p.Nu * p.ntile * kSlabTile;
+  a.uh = uh;
+  a.bl = blines;
+  a.hinv = hinv;
+  a.sa = sa;
+  a.sb = sb;
+  const long long warps = (long long)p.Nu * a.cur * p.L;
+  k_slice_lines<<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(a);
+  WLG_LAUNCH_CHECK("slice_lines");
+}
+
+void slice_gram(const SlicePlan& p, int chunk, unsigned char* sa, unsigned char* sb,
+                unsigned long long* acc, int* fail, cudaStream_t st) {
+  CUtensorMap ma, mb;
+  const long long un = (long long)p.mwlr * p.nuc;
+  if (!plane_map(&ma, sa, p.rows_a, un, 128) || !plane_map(&mb, sb, p.rows_b, un, p.TN)) {
+    set_error("kernel slice_gram: tensor map refused");
+    return;
+  }
+  GramTileArgs a;
+  a.N0 = p.N0;
+  a.Nu = p.Nu;
+  a.L = p.L;
+  a.mwlt = p.mwlt;
+  a.mwlr = p.mwlr;
+  a.rows_a = p.rows_a;
+  a.rows_b = p.rows_b;
+  a.TN = p.TN;
+  a.nmt = p.nmt;
+  a.ntiles = p.ntiles;
+  a.kstride = p.nuc * 9;
+  a.kcur = std::min(p.nuc, 3 * p.ntile - chunk * p.nuc) * 9;
+  a.kps = p.kps;
+  a.nsplit = p.nsplit;
+  a.stages = p.stages;
+  a.tmem_cols = (unsigned)p.tmem_cols;
+  a.nwl = (long long)p.nwl;
+  a.acc = acc;
+  a.fail = fail;
+  const long long items = (long long)p.mwlr * p.nsplit * p.ntiles;
+  const unsigned grid = (unsigned)std::min<long long>(items, num_sms());
+  void* args[] = {&ma, &mb, &a};
+  cudaLaunchKernel((void*)k_slice_gram, dim3(grid), dim3(kGramThreads), args, p.smem, st);
+  WLG_LAUNCH_CHECK("slice_gram");
+}
+
+void slice_finish(const Geo& g, const SlicePlan& p, int bc, const unsigned long long* acc,
+                  double* wl, cudaStream_t st) {
+  const double norm = 9.0 * g.n[1] * g.n[2] * g.n[3];  // wloop.c:535
+  const unsigned grid =
+      (unsigned)std::min<size_t>((p.nwl + 255) / 256, (size_t)num_sms() * 16);
+  const long long* s = reinterpret_cast<const long long*>(acc);
+  k_slice_finish<<<grid, 256, 0, st>>>(s, (long long)p.nwl, p.N0, p.mwlt, p.mwlr, p.L * p.L,
+                                       bc == 0, norm, wl);
+  WLG_LAUNCH_CHECK("slice_finish");
+}
+
+}  // namespace wlg

@@ -143,6 +143,7 @@ struct GramPlan {
 // upper bound), pipeline stages, column chunks per block.
 struct GramTuning {
   int occ = 0, ord = 0, bx = 0, stages = 0, cpc = 0;
+  bool set() const { return occ || ord || bx || stages || cpc; }
 };
 bool gram_plan(GramPlan& p, const Geo& g, int bc, int msl, int mwlt, bool fp64,
                const GramTuning* tune = nullptr);
@@ -185,6 +186,42 @@ void gram_contract(const Geo& g, const GramPlan& p, int mwlt, const T* alines, c
 template <class T>
 void gram_reduce(const Geo& g, const GramPlan& p, int bc, int mwlt, int mwlr, int r,
                  const T* partial, double* wl, cudaStream_t st);
+
+// ---- its FP64 Gram product as exact 8-bit digit products on the tensor cores
+// (gslice.cu) ----------------------------------------------------------------
+struct SlicePlan {
+  int L = 0, N0 = 0, Nu = 0, mwlt = 0, mwlr = 0, ntile = 0;
+  int rows_a = 0, rows_b = 0;     // rows (slice, level) of the A and B planes
+  int TN = 0, nmt = 0, ntiles = 0;  // B rows per tile, 128-row A tiles, tiles
+  int stages = 0, tmem_cols = 0;
+  size_t smem = 0;
+  int nuc = 0, nchunk = 0;        // column units per chunk, chunks
+  int kps = 0, nsplit = 0;        // K blocks per work item, column splits
+  size_t bytes_a = 0, bytes_b = 0, acc_bytes = 0, nwl = 0;
+};
+// device memory the digit planes of one chunk may take (false: one column unit
+// needs more)
+constexpr size_t kSliceBudget = (size_t)2 << 30;
+bool slice_plan(SlicePlan& p, const Geo& g, int bc, int msl, int mwlt, int mwlr,
+                size_t budget = kSliceBudget);
+// whether every line entry stays within the digits' range, from max |g g^dag - 1|
+// and max |U^dag U - 1| over the levels (false for NaN)
+bool slice_in_range(double dev, double delta, int mwlr);
+// shared-memory limit and driver entry point (before any launch or capture)
+int slice_prepare();
+// *dev (device): max |U^dag U - 1| over the msl levels, as double bits
+void levels_deviation(const Geo& g, int msl, const double2* levels,
+                      unsigned long long* dev, cudaStream_t st);
+// digit planes of one chunk for R = 1..mwlr from the first lines, the recursion
+// links and H^-1
+void slice_lines(const Geo& g, const SlicePlan& p, int chunk, const double* uh,
+                 const double* blines, const double* hinv, unsigned char* sa, unsigned char* sb, cudaStream_t st);
+// adds the chunk's sums to acc (zeroed before the first chunk); *fail set if a
+// wait ran out
+void slice_gram(const SlicePlan& p, int chunk, unsigned char* sa, unsigned char* sb,
+                unsigned long long* acc, int* fail, cudaStream_t st);
+void slice_finish(const Geo& g, const SlicePlan& p, int bc, const unsigned long long* acc,
+                  double* wl, cudaStream_t st);
 
 // ---- batched stages (one launch over many lattices) ------------------------
 // A: device array of n per-lattice argument records; pre: device array of

@@ -15,6 +15,7 @@
 // Every stage also has a batched kernel that covers many lattices in one
 // launch (flattened work list, find_item).
 #include "internal.h"
+#include "mbar.cuh"
 
 namespace wlg {
 
@@ -326,64 +327,6 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // Every wait is bounded: a wait that runs out sets g_stage_timeout,
 // which the host reads after the measurement.
 __device__ int g_stage_timeout;
-
-__device__ __forceinline__ unsigned smem_addr(const void* p) {
-  return (unsigned)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(count)
-               : "memory");
-}
-// before the barrier's shared memory goes back to other uses
-__device__ __forceinline__ void mbar_inval(uint64_t* bar) {
-  asm volatile("mbarrier.inval.shared::cta.b64 [%0];\n" ::"r"(smem_addr(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_init_fence() {
-  asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_addr(bar)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned phase) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_addr(bar)), "r"(phase)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %globaltimer;\n" : "=l"(t));
-  return t;
-}
-// waits at most limit_ns of wall time (the global nanosecond timer bounds it,
-// whatever each try_wait's own suspension); false if the phase did not complete
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned phase,
-                                                  uint64_t limit_ns = 2000000000ull) {
-  if (mbar_try_wait(bar, phase)) return true;
-  const uint64_t t0 = global_ns();
-  while (!mbar_try_wait(bar, phase))
-    if (global_ns() - t0 > limit_ns) return false;
-  return true;
-}
-// orders this thread's earlier shared-memory accesses before later
-// async-proxy (bulk copy) writes to the same memory
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-}
-// dst, src and bytes multiples of 16
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::
-          "r"(smem_addr(dst)),
-      "l"(src), "r"(bytes), "r"(smem_addr(bar))
-      : "memory");
-}
 
 // 16-byte chunk q of link s in a tiled direction array (common.cuh layout)
 template <class T> __device__ __forceinline__ const char* chunk_ptr(const typename V2<T>::t* base, int s, int q);
