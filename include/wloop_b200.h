@@ -297,9 +297,11 @@ int wlg_contract_form(wlg_ctx* ctx, int* form);
  * bx an upper bound on the start slices per block, stages the copy pipeline
  * depth (2-4), cpc the column chunks per block.  Results do not depend on
  * occ, ord, bx or stages; cpc sets how the FP32 sums of the mixed form are
- * split (FP32 rounding only).  In the FP64 form any of them asks for the FMA
- * kernel; with none, fields whose lines stay in the digits' range are
- * multiplied as exact 8-bit digits on the tensor cores. */
+ * split (FP32 rounding only).  Any of them asks for the kernel that runs one
+ * launch per spatial extent; with none, all extents run in one walk: the FP64
+ * form (fields whose lines stay in the digits' range) as exact 8-bit digit
+ * products on the tensor cores, the mixed form in packed FMAs, with the same
+ * result. */
 int wlg_set_gram_tuning(wlg_ctx* ctx, int occ, int ord, int bx, int stages, int cpc);
 /* The plan those settings give for msl levels and mwlt on ctx's lattice:
  * shape[10] = {extents per thread, occ, ord, start slices per block, blocks
@@ -324,6 +326,14 @@ int wlg_gram_plan_shape(const int n[4], int bc, int msl, int mwlt, int precision
  * planes may take (0: the default). */
 int wlg_slice_plan_shape(const int n[4], int bc, int msl, int mwlt, int mwlr, long long budget,
                          long long shape[16]);
+/* The plan of the mixed temporal-gauge form's packed-FMA Gram product (host
+ * only): level pairs, extents per thread, extent groups, start slices per block,
+ * padded to 8, staged B slices, blocks of start slices, stages, threads per
+ * block, blocks per SM, shared memory per block, column chunks per run, runs,
+ * chunks, runs per pass, passes, column units per pass, bytes of a pass's A and
+ * B lines and partial sums.  budget: bytes a pass may take (0: the default). */
+int wlg_pair_plan_shape(const int n[4], int bc, int msl, int mwlt, int mwlr, long long budget,
+                        long long shape[20]);
 /* The context's CUDA stream (cudaStream_t), for callers that record events. */
 void* wlg_stream(wlg_ctx* ctx);
 /* Number of wloop_b200 kernel launches issued by this process so far. */

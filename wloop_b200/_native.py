@@ -96,6 +96,7 @@ def _load():
         "wlg_gram_shape": (i, [vp, i, i, ip]),
         "wlg_gram_plan_shape": (i, [ip, i, i, i, i, ip, C.POINTER(C.c_longlong)]),
         "wlg_slice_plan_shape": (i, [ip, i, i, i, i, C.c_longlong, C.POINTER(C.c_longlong)]),
+        "wlg_pair_plan_shape": (i, [ip, i, i, i, i, C.c_longlong, C.POINTER(C.c_longlong)]),
         "wlg_launch_count": (C.c_longlong, []),
         "wlg_snapshot": (i, [vp]),
         "wlg_gauge_transform": (i, [vp, u64, d]),

@@ -52,12 +52,17 @@ struct Cfg {
   bool slices;
   SlicePlan sp;
   size_t gS, gAcc;
+  // the mixed form's packed Gram product (gpair.cu): its lines and partial sums
+  // take the level store too, or the scratch of the lattice's stream where the
+  // store is small and the scratch could be had
+  bool pairs, pairs_scratch;
+  PairPlan pp, pp_scratch;
   size_t gpartial;  // byte offset of its partial sums in the partial-sum buffer
 };
 
 enum OpKind {
   OP_SMEAR, OP_COPY, OP_LINES, OP_CONTRACT, OP_REDUCE, OP_D2H,
-  OP_GRAM_CHAIN, OP_GRAM_PREP, OP_GRAM_R, OP_SLICES
+  OP_GRAM_CHAIN, OP_GRAM_PREP, OP_GRAM_R, OP_SLICES, OP_PAIRS
 };
 
 struct Op {
@@ -76,6 +81,11 @@ struct Op {
 };
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
+
+// most a lattice stream's scratch takes: a small lattice's level store would cut
+// its loop stage into passes too short to fill the GPU (16^3x32 with 4 levels:
+// 126 MB, 17 passes)
+constexpr size_t kScratchBytes = (size_t)512 << 20;
 
 }  // namespace
 
@@ -104,8 +114,8 @@ struct wlg_batch {
     cudaGraphExec_t exec = nullptr;
     int kernels = 0;  // kernels one run of the phase launches
   } ph[2];
-  // per lattice, phase 1: 0 carried lines, 1 temporal gauge with the FMA Gram
-  // product, 2 with the tensor-core one
+  // per lattice, phase 1: 0 carried lines, 1 temporal gauge with one launch per
+  // extent, 2 with all extents in one walk (FP64: tensor cores; mixed: packed FMAs)
   std::vector<char> use_gram;
   bool use_graph = true;       // capture each phase after its first run and replay it
   int tG = 0, tSB = 0, tBlock = 0, tNCB = 0;  // contraction shape override (tuning)
@@ -116,6 +126,7 @@ struct wlg_batch {
   // different lattices overlap
   static constexpr int kSide = 4;
   cudaStream_t side[kSide] = {nullptr, nullptr, nullptr, nullptr};
+  char* scratch[kSide] = {nullptr, nullptr, nullptr, nullptr};
   cudaEvent_t fork = nullptr, join[kSide] = {nullptr, nullptr, nullptr, nullptr};
   float last_ms = 0.f;
   int kernels = 0;
@@ -385,7 +396,7 @@ template <class T> void build_ops(wlg_batch* b, int phase) {
   }
   cur_phase = 1;
   auto gram_on = [&](int c) { return c < (int)b->use_gram.size() && b->use_gram[c]; };
-  auto slices_on = [&](int c) { return gram_on(c) && b->use_gram[c] == 2; };
+  auto walk_on = [&](int c) { return gram_on(c) && b->use_gram[c] == 2; };
 
   // ---- loops (wloop.c:524-608) ----
   // temporal-gauge lattices: the first lines, then per R their line step,
@@ -393,13 +404,13 @@ template <class T> void build_ops(wlg_batch* b, int phase) {
   for (int c = 0; c < n; c++) {
     if (!gram_on(c)) continue;
     Op op{};
-    op.kind = slices_on(c) ? OP_SLICES : OP_GRAM_PREP;
+    op.kind = !walk_on(c) ? OP_GRAM_PREP : (b->cfg[c].slices ? OP_SLICES : OP_PAIRS);
     op.cfg = c;
     sink.push_back(op);
   }
   for (int r = 0; r < maxr; r++)
     for (int c = 0; c < n; c++) {
-      if (!gram_on(c) || slices_on(c) || r >= b->cfg[c].p.mwlr) continue;
+      if (!gram_on(c) || walk_on(c) || r >= b->cfg[c].p.mwlr) continue;
       Op op{};
       op.kind = OP_GRAM_R;
       op.cfg = c;
@@ -502,7 +513,7 @@ template <class T> void build_ops(wlg_batch* b, int phase) {
     }
   }
   for (int c = 0; c < n; c++) {
-    if (!slices_on(c)) continue;
+    if (!walk_on(c)) continue;
     Op op{};
     op.kind = OP_D2H;
     op.dst = b->dev_host + 3 * c + 2;
@@ -534,7 +545,8 @@ template <class T> int issue(wlg_batch* b, int phase) {
   };
   for (const Op& op : b->ph[phase].ops) {
     const bool gram_op =
-        op.kind == OP_GRAM_PREP || op.kind == OP_GRAM_R || op.kind == OP_SLICES;
+        op.kind == OP_GRAM_PREP || op.kind == OP_GRAM_R || op.kind == OP_SLICES ||
+        op.kind == OP_PAIRS;
     if (gram_op && !forked && b->side[0]) {
       WLG_CUDA(cudaEventRecord(b->fork, b->st));
       for (int k = 0; k < wlg_batch::kSide; k++) WLG_CUDA(cudaStreamWaitEvent(b->side[k], b->fork, 0));
@@ -612,6 +624,31 @@ template <class T> int issue(wlg_batch* b, int phase) {
         kernels += 2 + 2 * f.sp.nchunk;
         break;
       }
+      case OP_PAIRS: {
+        const Cfg& f = b->cfg[op.cfg];
+        const PairPlan& pp = f.pairs_scratch ? f.pp_scratch : f.pp;
+        cudaStream_t ls = lattice_stream(op.cfg);
+        float* uh = (float*)(b->arena + f.gUh);
+        float* bl = (float*)(b->arena + f.gB);
+        float* hf = (float*)(b->arena + f.gG);  // H^-1 in FP32 takes the place of g
+        const double* hinv = (const double*)(b->arena + f.gH);
+        gauge_first<float>(f.g, f.gp, f.p.msl,
+                           (const float2*)(b->arena + f.region + 6 * f.D * elem_bytes(b)),
+                           (const double*)(b->arena + f.gG), hinv, uh, bl, nullptr, ls);
+        narrow(hinv, hf, f.gp.A, ls);
+        char* pa = f.pairs_scratch ? b->scratch[op.cfg % wlg_batch::kSide] : b->arena + f.gS;
+        char* pb = pa + align256(pp.bytes_a);
+        float* part = (float*)(pb + align256(pp.bytes_b));
+        int* fail = (int*)((unsigned long long*)(b->arena + f.gDev) + 2);
+        WLG_CUDA(cudaMemsetAsync(fail, 0, sizeof(unsigned long long), ls));
+        for (int k = 0; k < pp.npass; k++) {
+          pair_lines(f.g, pp, k, uh, bl, hf, pa, pb, ls);
+          pair_gram(pp, k, pa, pb, part, fail, ls);
+          pair_reduce(f.g, pp, k, f.bc, part, (double*)(b->arena + f.wl), ls);
+        }
+        kernels += 2 + 3 * pp.npass;
+        break;
+      }
       case OP_GRAM_PREP: {
         const Cfg& f = b->cfg[op.cfg];
         typedef typename V2<T>::t T2;
@@ -671,6 +708,7 @@ int plan(wlg_batch* b) {
     // carried lines per lattice, so those get their partial sums too)
     f.gram = f.gram_ok && b->tG == 0;
     f.slices = f.gram && f.sp.nchunk > 0;
+    f.pairs = f.gram && (f.pp.npass > 0 || f.pairs_scratch);
     if (f.gram) {
       f.gpartial = poff;
       poff = align256(poff + f.gp.partial_elems * (fp64 ? 8 : 4));
@@ -735,6 +773,14 @@ void layout(wlg_batch* b) {
         o = align256(o + f.sp.acc_bytes);
       } else {
         f.sp = SlicePlan();
+      }
+      if (!fp64) {
+        if (room <= 1024 || !pair_plan(f.pp, f.gp, f.g, f.p.msl, f.p.mwlt, f.p.mwlr,
+                                       std::min(room - 1024, kPairBudget)))
+          f.pp = PairPlan();
+        if (room < kScratchBytes &&
+            !pair_plan(f.pp_scratch, f.gp, f.g, f.p.msl, f.p.mwlt, f.p.mwlr, kScratchBytes - 1024))
+          f.pp_scratch = PairPlan();
       }
       if (2 * gh <= 6 * f.D * es) {
         f.gG = f.region;
@@ -941,6 +987,23 @@ int wlg_batch_create(int nconf, const int* dims, const int* bcs, const wlg_wloop
     wlg_batch_destroy(b);
     return -1;
   }
+  // scratch of the lattice streams, where there is memory for it
+  for (int k = 0; k < wlg_batch::kSide; k++) {
+    size_t most = 0;
+    for (size_t c = k; c < b->cfg.size(); c += wlg_batch::kSide) {
+      const PairPlan& q = b->cfg[c].pp_scratch;
+      if (q.npass > 0)
+        most = std::max(most, align256(q.bytes_a) + align256(q.bytes_b) + align256(q.bytes_p));
+    }
+    if (most == 0 || pool_alloc(b, &b->scratch[k], most)) continue;
+    for (size_t c = k; c < b->cfg.size(); c += wlg_batch::kSide)
+      b->cfg[c].pairs_scratch = b->cfg[c].pp_scratch.npass > 0;
+  }
+  WLG_CUDA(cudaStreamSynchronize(b->st));
+  if (plan(b)) {
+    wlg_batch_destroy(b);
+    return -1;
+  }
   cudaEventCreate(&b->ev0);
   cudaEventCreate(&b->ev1);
   *out = b;
@@ -956,6 +1019,7 @@ int wlg_batch_destroy(wlg_batch* b) {
     pool_free(b, b->arena);
     pool_free(b, b->pbuf);
     pool_free(b, b->staging);
+    for (int k = 0; k < wlg_batch::kSide; k++) pool_free(b, b->scratch[k]);
     cudaStreamSynchronize(b->st);  // the frees are ordered on the stream
   }
   if (b->wl_host) cudaFreeHost(b->wl_host);
@@ -1088,8 +1152,9 @@ int wlg_batch_run(wlg_batch* b) {
     double dev[2];
     memcpy(dev, b->dev_host + 3 * c, sizeof(dev));
     use[c] = dev[0] <= kGramMaxDeviation;
-    if (use[c] && b->cfg[c].slices && slice_in_range(dev[0], dev[1], b->cfg[c].p.mwlr) &&
-        slice_prepare() == 0)
+    const Cfg& f = b->cfg[c];
+    if (use[c] && ((f.slices && slice_in_range(dev[0], dev[1], f.p.mwlr) && slice_prepare() == 0) ||
+                   (f.pairs && pair_prepare(f.pairs_scratch ? f.pp_scratch : f.pp) == 0)))
       use[c] = 2;
     set_error("%s", "");
   }

@@ -69,7 +69,8 @@ struct wlg_ctx {
   // the temporal-gauge form: g, H^-1, recursion links, B and A lines, the
   // unitarity deviation of g
   DevBuf gG, gH, gUh, gB, gA, gDev;
-  // its tensor-core Gram product: digit planes, integer sums
+  // the lines of one chunk of columns, all extents (digit planes or FP32 level
+  // pairs), and the tensor-core product's integer sums
   DevBuf gSa, gSb, gAcc;
   void* lines_at = nullptr;  // buffer holding the lines of length lines_len
   // after a temporal-gauge measurement the lines of length lines_lazy are
@@ -464,6 +465,73 @@ static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan&
   return 0;
 }
 
+// The mixed form's loop stage in packed FMAs (gpair.cu), once g and H^-1 exist:
+// the first lines, then per pass of column runs the lines of every R, their
+// Gram products and the runs' sums.  Returns 1 (nothing done) when its buffers
+// do not fit.
+static int do_loops_pairs(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan& gp,
+                          const PairPlan& pp, double* wl_mat) {
+  const Geo& g = c->g;
+  const int msl = p->msl;
+  const size_t nb = gp.A * sizeof(float) * 3 * msl;
+  const size_t nwl = (size_t)msl * msl * p->mwlt * p->mwlr * g.n[0];
+  auto alloc = [&]() {
+    return ensure(c->gUh, nb) || ensure(c->gB, nb) || ensure(c->gSa, pp.bytes_a) ||
+           ensure(c->gSb, pp.bytes_b) || ensure(c->partial, pp.bytes_p) ||
+           ensure(c->wl, sizeof(double) * nwl);
+  };
+  if (alloc()) {
+    release_idle_scratch(c);
+    if (alloc()) {
+      set_error("%s", "");
+      release(c->gSa);
+      release(c->gSb);
+      return 1;
+    }
+  }
+  c->used_variant = 11;
+  c->lines_len = 0;
+  c->lines_at = nullptr;
+  c->lines_lazy = p->mwlr >= 2 ? p->mwlr : 0;
+  float* uh = (float*)c->gUh.p;
+  float* bl = (float*)c->gB.p;
+  const double* hinv = (const double*)c->gH.p;
+  float* hf = (float*)c->gG.p;  // H^-1 in FP32 takes the place of g, dead by then
+  int* fail = (int*)((unsigned long long*)c->gDev.p + 2);
+  WLG_CUDA(cudaMemsetAsync(fail, 0, sizeof(int), c->st));
+  {
+    ProfScope ps(c, "gauge");
+    gauge_first<float>(g, gp, msl, (const float2*)c->levels.p, (const double*)c->gG.p, hinv, uh, bl,
+                       nullptr, c->st);
+    narrow(hinv, hf, gp.A, c->st);
+  }
+  for (int k = 0; k < pp.npass; k++) {
+    {
+      ProfScope ps(c, "lines");
+      pair_lines(g, pp, k, uh, bl, hf, c->gSa.p, c->gSb.p, c->st);
+    }
+    {
+      ProfScope ps(c, "contract");
+      pair_gram(pp, k, c->gSa.p, c->gSb.p, (float*)c->partial.p, fail, c->st);
+    }
+    {
+      ProfScope ps(c, "reduce");
+      pair_reduce(g, pp, k, c->bc, (const float*)c->partial.p, (double*)c->wl.p, c->st);
+    }
+  }
+  if (get_error()[0]) return -1;
+  int failed = 0;
+  WLG_CUDA(cudaMemcpyAsync(&failed, fail, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+  if (wl_mat)
+    WLG_CUDA(cudaMemcpyAsync(wl_mat, c->wl.p, sizeof(double) * nwl, cudaMemcpyDeviceToHost, c->st));
+  WLG_CUDA(cudaStreamSynchronize(c->st));
+  if (failed) {
+    set_error("wloop_sum: the Gram product's operand copies did not arrive in time");
+    return -1;
+  }
+  return 0;
+}
+
 // wloops() in the temporal gauge (gram.cu): the gauge field and H^-1 once,
 // then the first lines; per R the line step, the banded Gram product and its
 // reduction.  Returns 1 (nothing done) when the form does not apply: shapes
@@ -485,6 +553,9 @@ static int do_loops_gram(wlg_ctx* c, const wlg_wloop_parms* p, double* wl_mat) {
   // a tuned shape asks for the FMA kernel
   bool slices = fp64 && !c->gtune.set() && slice_plan(sp, g, c->bc, msl, p->mwlt, p->mwlr) &&
                 slice_prepare() == 0;
+  PairPlan pp;
+  const bool pairs = !fp64 && !c->gtune.set() &&
+                     pair_plan(pp, gp, g, msl, p->mwlt, p->mwlr) && pair_prepare(pp) == 0;
   if (gram_prepare(gp)) return -1;
   const size_t nb = gp.A * sizeof(T) * 3 * msl, na = gp.Aa * sizeof(T) * 3 * msl;
   const size_t nwl = (size_t)msl * msl * p->mwlt * p->mwlr * g.n[0];
@@ -505,6 +576,10 @@ static int do_loops_gram(wlg_ctx* c, const wlg_wloop_parms* p, double* wl_mat) {
   slices = slices && slice_in_range(dev[0], dev[1], p->mwlr);
   if (slices) {
     const int rc = do_loops_slices(c, p, gp, sp, wl_mat);
+    if (rc != 1) return rc;
+  }
+  if (pairs) {
+    const int rc = do_loops_pairs(c, p, gp, pp, wl_mat);
     if (rc != 1) return rc;
   }
   auto alloc = [&]() {
@@ -1342,6 +1417,38 @@ int wlg_slice_plan_shape(const int n[4], int bc, int msl, int mwlt, int mwlr, lo
                            (long long)sp.bytes_a, (long long)sp.bytes_b, (long long)sp.acc_bytes,
                            sp.ntile};
   for (int i = 0; i < 16; i++) shape[i] = v[i];
+  return 0;
+}
+
+int wlg_pair_plan_shape(const int n[4], int bc, int msl, int mwlt, int mwlr, long long budget,
+                        long long shape[20]) {
+  set_error("%s", "");
+  if (!n || !shape || (bc != 0 && bc != 3) || budget < 0) {
+    set_error("pair_plan_shape: bad arguments");
+    return -1;
+  }
+  for (int i = 0; i < 4; i++)
+    if (n[i] < 2) {
+      set_error("pair_plan_shape: lattice extent N%d=%d < 2", i, n[i]);
+      return -1;
+    }
+  if ((long long)n[0] * n[1] * n[2] * n[3] > (1LL << 30)) {
+    set_error("pair_plan_shape: lattice volume too large");
+    return -1;
+  }
+  const Geo g = make_geo(n);
+  GramPlan gp;
+  PairPlan pp;
+  if (!gram_plan(gp, g, bc, msl, mwlt, false) ||
+      !pair_plan(pp, gp, g, msl, mwlt, mwlr, budget ? (size_t)budget : kPairBudget)) {
+    set_error("no level-pair plan for msl %d, mwlt %d, mwlr %d", msl, mwlt, mwlr);
+    return -1;
+  }
+  const long long v[20] = {pp.LP, pp.TQ, pp.NG, pp.BX, pp.BXp, pp.NYBp, pp.nblk, pp.stages,
+                           pp.block, pp.ctas, (long long)pp.smem, pp.cpc, pp.nsplit, pp.nchunks,
+                           pp.runs, pp.npass, pp.nuc, (long long)pp.bytes_a,
+                           (long long)pp.bytes_b, (long long)pp.bytes_p};
+  for (int i = 0; i < 20; i++) shape[i] = v[i];
   return 0;
 }
 

@@ -39,8 +39,6 @@
 // in any order): a lane writes 16 bytes and 2 bytes per plane at offsets the
 // compiler knows, a warp one contiguous row, and an operand tile (rows x
 // planes of one K block) is one TMA box.
-#include <cuda.h>
-
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -50,6 +48,7 @@
 #include "internal.h"
 #include "mbar.cuh"
 #include "slab.cuh"
+#include "tensormap.h"
 
 namespace wlg {
 namespace {
@@ -307,9 +306,6 @@ __device__ __forceinline__ void tc_fence_after() {
 __device__ __forceinline__ void tc_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_addr(bar)) : "memory");
-}
 __device__ __forceinline__ void tmem_ld16(int (&v)[16], unsigned addr) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -321,20 +317,6 @@ __device__ __forceinline__ void tmem_ld16(int (&v)[16], unsigned addr) {
 }
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-}
-
-// bounded wait that also ends when another role has given up
-__device__ __forceinline__ bool wait_or_quit(uint64_t* bar, unsigned phase, volatile int* quit) {
-  if (mbar_try_wait(bar, phase)) return true;
-  const uint64_t t0 = global_ns();
-  while (!mbar_try_wait(bar, phase)) {
-    if (*quit) return false;
-    if (global_ns() - t0 > 2000000000ull) {
-      *quit = 1;
-      return false;
-    }
-  }
-  return true;
 }
 
 __global__ void __launch_bounds__(kGramThreads, 1)
@@ -561,31 +543,11 @@ constexpr size_t kSmemMax = 227 * 1024 - 1024;  // beside the barriers and the a
 // at most 2^14 a column, 64 columns a block
 constexpr int kRunMax = (int)((1ll << 31) / ((long long)kPlanes * (1 << 14) * kKB)) - 1;
 
-typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                             const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                             CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                             CUtensorMapFloatOOBfill);
-
-EncodeFn encode_fn() {
-  static EncodeFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult res;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault,
-                                         &res) != cudaSuccess ||
-        res != cudaDriverEntryPointSuccess) {
-      cudaGetLastError();
-      p = nullptr;
-    }
-    return (EncodeFn)p;
-  }();
-  return fn;
-}
-
 // planes as a tensor of (64 bytes, rows, planes, blocks, (R, unit)); box: `box`
 // rows of all planes of one K block
 bool plane_map(CUtensorMap* m, void* base, int rows, long long units, int box) {
   constexpr int P = kPlanes;
-  EncodeFn fn = encode_fn();
+  TensorMapEncode fn = tensor_map_encode();
   if (!fn) return false;
   const cuuint64_t pitch = (cuuint64_t)9 * P * kKB;
   const cuuint64_t dim[5] = {kKB, (cuuint64_t)rows, (cuuint64_t)P, 9, (cuuint64_t)units};
@@ -680,7 +642,7 @@ int slice_prepare() {
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lock(mu);
   if (done.count({dev, fn})) return 0;
-  if (!encode_fn()) {
+  if (!tensor_map_encode()) {
     set_error("slice gram: the driver has no cuTensorMapEncodeTiled");
     return -1;
   }

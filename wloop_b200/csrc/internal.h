@@ -223,6 +223,36 @@ void slice_gram(const SlicePlan& p, int chunk, unsigned char* sa, unsigned char*
 void slice_finish(const Geo& g, const SlicePlan& p, int bc, const unsigned long long* acc,
                   double* wl, cudaStream_t st);
 
+// ---- its mixed-form Gram product in packed FMAs, all extents in one walk
+// (gpair.cu); the runs of columns are those of the GramPlan it is made from ----
+struct PairPlan {
+  int L = 0, LP = 0, N0 = 0, Nu = 0, ntile = 0, mwlt = 0, mwlr = 0;
+  int cpc = 0, nsplit = 0, nchunks = 0;  // chunks per run, runs, chunks (GramPlan)
+  int TQ = 0, NG = 0, BX = 0, BXp = 0, NYBp = 0, nblk = 0, stages = 0, block = 0;
+  int ctas = 0;                          // CTAs per SM
+  size_t smem = 0;
+  int runs = 0, npass = 0, nuc = 0;      // runs per pass, passes, column units per pass
+  size_t bytes_a = 0, bytes_b = 0, bytes_p = 0;  // A and B lines, partial sums of a pass
+};
+// device memory the lines and partial sums of one pass may take (false: one run
+// needs more)
+constexpr size_t kPairBudget = (size_t)4 << 30;
+bool pair_plan(PairPlan& p, const GramPlan& gp, const Geo& g, int msl, int mwlt, int mwlr,
+               size_t budget = kPairBudget);
+int pair_prepare(const PairPlan& p);
+// n doubles of H^-1 as floats
+void narrow(const double* src, float* dst, size_t n, cudaStream_t st);
+// lines of one pass for R = 1..mwlr from the first lines, the recursion links
+// and H^-1
+void pair_lines(const Geo& g, const PairPlan& p, int pass, const float* uh, const float* blines,
+                const float* hinv, void* pa, void* pb, cudaStream_t st);
+// partial sums of the pass; *fail set if a wait ran out
+void pair_gram(const PairPlan& p, int pass, void* pa, void* pb, float* partial, int* fail,
+               cudaStream_t st);
+// adds them to wl; the passes in order
+void pair_reduce(const Geo& g, const PairPlan& p, int pass, int bc, const float* partial, double* wl,
+                 cudaStream_t st);
+
 // ---- batched stages (one launch over many lattices) ------------------------
 // A: device array of n per-lattice argument records; pre: device array of
 // n+1 prefix sums of the per-lattice work items (blocks for the contraction).

@@ -49,6 +49,22 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned phase,
     if (global_ns() - t0 > limit_ns) return false;
   return true;
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_addr(bar)) : "memory");
+}
+// bounded wait that also ends when another role has given up
+__device__ __forceinline__ bool wait_or_quit(uint64_t* bar, unsigned phase, volatile int* quit) {
+  if (mbar_try_wait(bar, phase)) return true;
+  const uint64_t t0 = global_ns();
+  while (!mbar_try_wait(bar, phase)) {
+    if (*quit) return false;
+    if (global_ns() - t0 > 2000000000ull) {
+      *quit = 1;
+      return false;
+    }
+  }
+  return true;
+}
 // orders this thread's earlier shared-memory accesses before later
 // async-proxy (bulk copy) writes to the same memory
 __device__ __forceinline__ void fence_proxy_async_smem() {
