@@ -51,7 +51,7 @@ def test_plans(n):
             assert p["nuc"] * p["nchunk"] >= units > p["nuc"] * (p["nchunk"] - 1)
             assert p["kps"] * p["nsplit"] >= 9 * p["nuc"] > p["kps"] * (p["nsplit"] - 1)
             assert p["kps"] * 64 * P * 128 * 128 < 2 ** 31
-            row = 9 * P * 64
+            row = 4096  # 9 x 7 x 64 digits, padded
             assert p["bytes_a"] == r * p["nuc"] * p["rows_a"] * row
             assert p["bytes_b"] == r * p["nuc"] * p["rows_b"] * row
             assert p["bytes_a"] + p["bytes_b"] <= 2 << 30

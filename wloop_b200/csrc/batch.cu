@@ -1153,7 +1153,7 @@ int wlg_batch_run(wlg_batch* b) {
     memcpy(dev, b->dev_host + 3 * c, sizeof(dev));
     use[c] = dev[0] <= kGramMaxDeviation;
     const Cfg& f = b->cfg[c];
-    if (use[c] && ((f.slices && slice_in_range(dev[0], dev[1], f.p.mwlr) && slice_prepare() == 0) ||
+    if (use[c] && ((f.slices && slice_in_range(dev[0], dev[1], f.p.mwlr) && slice_prepare(f.sp) == 0) ||
                    (f.pairs && pair_prepare(f.pairs_scratch ? f.pp_scratch : f.pp) == 0)))
       use[c] = 2;
     set_error("%s", "");

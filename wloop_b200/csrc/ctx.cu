@@ -552,7 +552,7 @@ static int do_loops_gram(wlg_ctx* c, const wlg_wloop_parms* p, double* wl_mat) {
   if (!fma_ok) return 1;
   // a tuned shape asks for the FMA kernel
   bool slices = fp64 && !c->gtune.set() && slice_plan(sp, g, c->bc, msl, p->mwlt, p->mwlr) &&
-                slice_prepare() == 0;
+                slice_prepare(sp) == 0;
   PairPlan pp;
   const bool pairs = !fp64 && !c->gtune.set() &&
                      pair_plan(pp, gp, g, msl, p->mwlt, p->mwlr) && pair_prepare(pp) == 0;

@@ -32,13 +32,15 @@
 //
 // Plane layout, one buffer for the A rows (start slice, level) and one for the
 // B rows (unrolled slice, level), row = slice * L + level: per (R, unit, row)
-// the P x 576 digits of one 32-site tile as 9 K blocks of 64 columns,
-//     byte (((r * nuc + unit) * rows + row) * 9 + b) * P * 64 + p * 64 + i
-// where block b < 8 holds the first 16 components of lanes 4 b .. 4 b + 3 and
-// block 8 the last two components of all lanes (the columns of a sum may come
-// in any order): a lane writes 16 bytes and 2 bytes per plane at offsets the
-// compiler knows, a warp one contiguous row, and an operand tile (rows x
-// planes of one K block) is one TMA box.
+// 4096 bytes that hold the 7 x 576 digits of one 32-site tile as 9 K blocks of
+// 64 columns, planes 0 .. 5 in pairs so that an operand row is a whole 128-byte
+// line (TMA moves about one row in 2.4 cycles, of 64 or of 128 bytes):
+//     plane p < 6 of block b at  b * 384 + (p / 2) * 128 + (p % 2) * 64
+//     plane 6 of block b at      3456 + b * 64
+// Block b < 8 holds the first 16 components of lanes 4 b .. 4 b + 3 and block
+// 8 the last two components of all lanes (the columns of a sum may come in any
+// order): a lane writes 16 bytes and 2 bytes per plane at offsets the compiler
+// knows, a warp one contiguous row.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -54,7 +56,9 @@ namespace wlg {
 namespace {
 
 constexpr int kPlanes = 7;
-constexpr int kKB = 64;       // bytes (columns) per K block: 32 sites x {re, im} of one entry
+constexpr int kKB = 64;       // bytes (columns) per K block
+constexpr int kRow = 4096;    // bytes of one row of planes
+constexpr int kSingle = 9 * 6 * kKB;  // where plane 6 starts in it
 constexpr int kMaxStages = 8;
 constexpr int kGramThreads = 192;  // producer warp, MMA warp, four epilogue warps
 
@@ -96,11 +100,13 @@ struct Digits {
   static constexpr unsigned flip(int p) { return p == 0 ? 0u : 0x80808080u; }
 };
 
+// where plane p starts in a lane's 16-byte (o6 for plane 6: o16) column
+__device__ constexpr int plane_at(int p) { return (p >> 1) * 128 + (p & 1) * kKB; }
+
 // the digit planes of one matrix into its row (this lane's 16 + 2 bytes per
 // plane); lanes without a site write zeros
-__device__ __forceinline__ void store_digits(unsigned char* __restrict__ o16,
-                                             unsigned char* __restrict__ o2, const M3<double>& m,
-                                             bool live) {
+__device__ __forceinline__ void store_digits(unsigned char* __restrict__ row, int lane,
+                                             const M3<double>& m, bool live) {
   constexpr int P = kPlanes;
   uint4 q[P];
 #pragma unroll
@@ -121,11 +127,16 @@ __device__ __forceinline__ void store_digits(unsigned char* __restrict__ o16,
   }
   unsigned w[P];
   Digits::half(w, Digits::raw(m.e[8]));
+  unsigned char* o16 = row + (lane >> 2) * (6 * kKB) + (lane & 3) * 16;
+  unsigned char* s16 = row + kSingle + lane * 16;
+  unsigned char* o2 = row + 8 * 6 * kKB + lane * 2;
+  unsigned char* s2 = row + kSingle + 8 * kKB + lane * 2;
 #pragma unroll
   for (int p = 0; p < P; p++) {
-    *reinterpret_cast<uint4*>(o16 + p * kKB) = q[p];
+    *reinterpret_cast<uint4*>(p < 6 ? o16 + plane_at(p) : s16) = q[p];
     const unsigned v = w[p] ^ (Digits::flip(p) & 0xffffu);
-    *reinterpret_cast<unsigned short*>(o2 + p * kKB) = (unsigned short)(live ? v : 0u);
+    *reinterpret_cast<unsigned short*>(p < 6 ? o2 + plane_at(p) : s2) =
+        (unsigned short)(live ? v : 0u);
   }
 }
 
@@ -154,8 +165,6 @@ struct LineArgs {
 // digit planes.  One warp per (y0, unit, level), levels in neighbouring warps
 // (they share the H^-1 tiles), the walk over R in registers.
 __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
-  constexpr int P = kPlanes;
-  constexpr int PITCH = 9 * P * kKB;  // bytes of one row
   const int lane = threadIdx.x & 31;
   unsigned w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lev = (int)(w % a.msl);
@@ -178,11 +187,9 @@ __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
   int z = j, y = (j / st) % nk;  // x + (R - 1) k and its coordinate along k
   const size_t rows_a = (size_t)g.n[0] * a.msl, rows_b = (size_t)a.Nu * a.msl;
   const int row = y0 * a.msl + lev;
-  const unsigned at16 = (unsigned)((lane >> 2) * P * kKB + (lane & 3) * 16);
-  const unsigned at2 = (unsigned)(8 * P * kKB + lane * 2);
-  unsigned char* ob = a.sb + (ul * rows_b + row) * PITCH;
-  unsigned char* oa = a.sa + (ul * rows_a + row) * PITCH;
-  const size_t step_b = a.nuc * rows_b * PITCH, step_a = a.nuc * rows_a * PITCH;
+  unsigned char* ob = a.sb + (ul * rows_b + row) * kRow;
+  unsigned char* oa = a.sa + (ul * rows_a + row) * kRow;
+  const size_t step_b = a.nuc * rows_b * kRow, step_a = a.nuc * rows_a * kRow;
   M3<double> c, f, t;
   ld_slab_as(c, a.bl + (size_t)(lev * 3 + k) * a.A + slice, j >> 5, j & 31);
 #pragma unroll 1
@@ -197,14 +204,14 @@ __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
       y = 0;
       z -= nk * st;
     }
-    store_digits(ob + at16, ob + at2, c, live);
+    store_digits(ob, lane, c, live);
     if (start) {
       ld_slab_as(f, hinv, z >> 5, z & 31);
       mul(t, c, f);
       ld_slab_as(f, hinv, j >> 5, j & 31);
       M3<double> s;
       mul(s, f, t);
-      store_digits(oa + at16, oa + at2, s, live);
+      store_digits(oa, lane, s, live);
     }
     ob += step_b;
     oa += step_a;
@@ -215,12 +222,15 @@ __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
 // The banded Gram product of one chunk.  A work item is (R, column split,
 // tile); a tile is 128 A rows against TN of the B rows their band reaches.
 // One CTA per SM walks items; per 64-column block the producer thread fetches
-// the P x 128 and P x TN digit rows with two TMA boxes (64-byte swizzle), the
-// MMA thread issues the digit pairs i + j < P, the pairs of one A plane with
-// neighbouring B planes as one MMA of up to 256 columns (their accumulators,
-// the classes i + j, are neighbours in TMEM too), and the epilogue warps read
-// the classes, combine them as 64-bit integers and add the entries inside the
-// band to the result with integer atomics.  Every wait is bounded: one that
+// the digit rows of both operands with four TMA boxes, the MMA thread issues
+// the digit pairs i + j < 7, one A plane with up to three B planes per MMA
+// (their accumulators, the classes i + j, are neighbours in TMEM), and the
+// epilogue warps read the classes, combine them as 64-bit integers and add the
+// entries inside the band to the result with integer atomics.  At 32^3x64 the
+// tensor pipe is 77 % busy (85 % with its set-up) at the 1.66 GHz the power
+// limit leaves: 70 ms a measurement; 84 ms with one 64-byte row per plane and
+// descriptors worked out by the issuing thread, 102 ms with a ring of single A
+// planes (two more blocks in flight, but seven boxes a block).  Every wait is bounded: one that
 // runs out sets *fail, and all roles leave.
 // ---------------------------------------------------------------------------
 struct GramTileArgs {
@@ -272,20 +282,36 @@ __device__ __forceinline__ TileAt tile_at(const GramTileArgs& a, long long it) {
   return t;
 }
 
-__device__ __forceinline__ void tma_box(unsigned dst, const CUtensorMap* map, int row, int b, int u,
-                                        uint64_t* bar) {
+__device__ __forceinline__ void tma_pairs(unsigned dst, const CUtensorMap* map, int row, int b,
+                                          int u, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
       "[%0], [%1, {%2, %3, %2, %4, %5}], [%6];\n" ::"r"(dst),
       "l"(map), "r"(0), "r"(row), "r"(b), "r"(u), "r"(smem_addr(bar))
       : "memory");
 }
+__device__ __forceinline__ void tma_single(unsigned dst, const CUtensorMap* map, int row, int b,
+                                           int u, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(dst),
+      "l"(map), "r"(0), "r"(row), "r"(b), "r"(u), "r"(smem_addr(bar))
+      : "memory");
+}
 
-// K-major shared-memory operand with 64-byte swizzle: 8-row groups of 512 bytes
-__device__ __forceinline__ uint64_t operand_desc(unsigned addr) {
+// K-major shared-memory operands: 8-row groups of 1024 bytes with 128-byte
+// swizzle (plane pairs), of 512 bytes with 64-byte swizzle (plane 6)
+__device__ __forceinline__ uint64_t pair_desc(unsigned addr) {
+  return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
+         ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+__device__ __forceinline__ uint64_t single_desc(unsigned addr) {
   return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)1 << 16) | ((uint64_t)(512 >> 4) << 32) |
          ((uint64_t)1 << 46) | ((uint64_t)4 << 61);
 }
+// TMEM column (in units of TN) of class m: the even classes, then the odd ones,
+// so that the classes of one A plane and B planes j, j + 2, ... are neighbours
+__host__ __device__ constexpr int class_col(int m) { return (m & 1) ? 4 + m / 2 : m / 2; }
 
 __device__ __forceinline__ void mma_i8(unsigned d, uint64_t da, uint64_t db, unsigned idesc,
                                        bool accumulate) {
@@ -319,8 +345,10 @@ __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
+template <int TN>
 __global__ void __launch_bounds__(kGramThreads, 1)
-    k_slice_gram(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+    k_slice_gram(const __grid_constant__ CUtensorMap map_a2, const __grid_constant__ CUtensorMap map_a1,
+                 const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ CUtensorMap map_b1,
                  const GramTileArgs a) {
   constexpr int P = kPlanes;
   extern __shared__ unsigned char raw[];
@@ -329,8 +357,9 @@ __global__ void __launch_bounds__(kGramThreads, 1)
   __shared__ int quit;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned base = (smem_addr(raw) + 1023u) & ~1023u;
-  const unsigned bytes_a = P * 128 * kKB, bytes_b = (unsigned)(P * a.TN * kKB);
-  const unsigned stage_bytes = bytes_a + bytes_b;
+  // a stage: A pairs, B pairs, A plane 6, B plane 6
+  constexpr unsigned at_b2 = 3 * 128 * 128, at_a1 = at_b2 + 3 * TN * 128, at_b1 = at_a1 + 128 * kKB;
+  constexpr unsigned stage_bytes = at_b1 + TN * kKB;
   if (threadIdx.x == 0) {
     for (int s = 0; s < a.stages; s++) {
       mbar_init(full + s, 1);
@@ -364,15 +393,14 @@ __global__ void __launch_bounds__(kGramThreads, 1)
       for (long long it = blockIdx.x; ok && it < items; it += gridDim.x) {
         const TileAt t = tile_at(a, it);
         for (int kb = 0; kb < t.nkb; kb++) {
-          if (!wait_or_quit(empty + s, ph ^ 1, &quit)) {
-            ok = false;
-            break;
-          }
+          if (!(ok = wait_or_quit(empty + s, ph ^ 1, &quit))) break;
           const unsigned dst = base + s * stage_bytes;
           mbar_expect_tx(full + s, stage_bytes);
           const int un = (t.kb0 + kb) / 9, bl = t.kb0 + kb - un * 9;
-          tma_box(dst, &map_a, t.m0, bl, un, full + s);
-          tma_box(dst + bytes_a, &map_b, t.b0, bl, un, full + s);
+          tma_pairs(dst, &map_a2, t.m0, bl, un, full + s);
+          tma_pairs(dst + at_b2, &map_b2, t.b0, bl, un, full + s);
+          tma_single(dst + at_a1, &map_a1, t.m0, bl, un, full + s);
+          tma_single(dst + at_b1, &map_b1, t.b0, bl, un, full + s);
           issued++;
           if (++s == a.stages) {
             s = 0;
@@ -391,28 +419,42 @@ __global__ void __launch_bounds__(kGramThreads, 1)
       int s = 0;
       unsigned ph = 0, aph = 0;
       bool ok = true;
-      const int gp = 256 / a.TN;  // B planes one MMA covers
-      const unsigned idesc0 = (2u << 4) | (1u << 7) | (1u << 10) | (8u << 24);  // S32, S8 x S8, M 128
+      constexpr unsigned idesc0 =
+          (2u << 4) | (1u << 7) | (1u << 10) | (8u << 24);  // S32, S8 x S8, M 128
       for (long long it = blockIdx.x; ok && it < items; it += gridDim.x) {
         const TileAt t = tile_at(a, it);
         if (t.nkb <= 0) continue;
         if (!(ok = wait_or_quit(&acc_empty, aph ^ 1, &quit))) break;
         tc_fence_after();
-        for (int kb = 0; kb < t.nkb; kb++) {
+        for (int kb = 0; ok && kb < t.nkb; kb++) {
           if (!(ok = wait_or_quit(full + s, ph, &quit))) break;
           tc_fence_after();
-          const unsigned sa = base + s * stage_bytes, sb = sa + bytes_a;
+          const unsigned sa = base + s * stage_bytes;
+          const uint64_t a2 = pair_desc(sa), b2 = pair_desc(sa + at_b2);
+          const uint64_t a1 = single_desc(sa + at_a1), b1 = single_desc(sa + at_b1);
+          // everything but the base addresses is known here: one thread issues
+          // all MMAs of the block.  A plane i against the B planes of one
+          // parity, j + i < 7, which lie one below the other: one MMA of up to
+          // 3 TN columns; plane 6 only meets plane 0.
 #pragma unroll
           for (int ks = 0; ks < kKB / 32; ks++)
 #pragma unroll
             for (int i = 0; i < P; i++) {
-              const uint64_t da = operand_desc(sa + i * 128 * kKB + ks * 32);
-              for (int jp = 0; jp < P - i; jp += gp) {
-                const int n = min(gp, P - i - jp) * a.TN;
-                mma_i8(tmem + (unsigned)((i + jp) * a.TN), da,
-                       operand_desc(sb + (unsigned)(jp * a.TN) * kKB + ks * 32),
-                       idesc0 | ((unsigned)(n >> 3) << 17), kb > 0 || ks > 0 || i > 0);
+              const bool acc = kb > 0 || ks > 0 || i > 0;
+              const uint64_t da = i < 6 ? a2 + (uint64_t)(((i >> 1) * 128 * 128 + (i & 1) * kKB + ks * 32) >> 4)
+                                        : a1 + (uint64_t)(ks * 32 >> 4);
+#pragma unroll
+              for (int h = 0; h < 2; h++) {
+                const int last = i == 0 ? 5 : 6 - i;
+                const int n = last < h ? 0 : (last - h) / 2 + 1;
+                if (n > 0)
+                  mma_i8(tmem + (unsigned)(class_col(i + h) * TN), da,
+                         b2 + (uint64_t)((h * kKB + ks * 32) >> 4),
+                         idesc0 | ((unsigned)(n * TN >> 3) << 17), acc);
               }
+              if (i == 0)
+                mma_i8(tmem + (unsigned)(class_col(6) * TN), da, b1 + (uint64_t)(ks * 32 >> 4),
+                       idesc0 | ((unsigned)(TN >> 3) << 17), acc);
             }
           mma_commit(empty + s);
           if (++s == a.stages) {
@@ -443,14 +485,14 @@ __global__ void __launch_bounds__(kGramThreads, 1)
         const int row = r0 + lane, x0 = row / a.L, s1 = row - x0 * a.L;
         // the columns any row of this warp needs
         const int lo = max(0, (r0 / a.L + 1) * a.L - t.b0);
-        const int hi = min(min(a.TN, a.rows_b - t.b0),
+        const int hi = min(min(TN, a.rows_b - t.b0),
                            (min(r0 + 31, a.rows_a - 1) / a.L + a.mwlt + 1) * a.L - t.b0);
         const bool live = row < a.rows_a;
         for (int c0 = lo & ~15; c0 < hi; c0 += 16) {
           int v[P][16];
 #pragma unroll
           for (int m = 0; m < P; m++)
-            tmem_ld16(v[m], tmem + ((unsigned)(quad * 32) << 16) + (unsigned)(m * a.TN + c0));
+            tmem_ld16(v[m], tmem + ((unsigned)(quad * 32) << 16) + (unsigned)(class_col(m) * TN + c0));
           tmem_ld_wait();
           int e = (t.b0 + c0) / a.L, s2 = t.b0 + c0 - e * a.L;
 #pragma unroll
@@ -543,22 +585,38 @@ constexpr size_t kSmemMax = 227 * 1024 - 1024;  // beside the barriers and the a
 // at most 2^14 a column, 64 columns a block
 constexpr int kRunMax = (int)((1ll << 31) / ((long long)kPlanes * (1 << 14) * kKB)) - 1;
 
-// planes as a tensor of (64 bytes, rows, planes, blocks, (R, unit)); box: `box`
-// rows of all planes of one K block
-bool plane_map(CUtensorMap* m, void* base, int rows, long long units, int box) {
-  constexpr int P = kPlanes;
+// plane pairs as a tensor of (128 bytes, rows, pairs, blocks, (R, unit)), plane 6
+// as one of (64 bytes, rows, blocks, (R, unit)); a box is `box` rows of one block
+bool plane_maps(CUtensorMap* pairs, CUtensorMap* single, unsigned char* base, int rows,
+                long long units, int box) {
   TensorMapEncode fn = tensor_map_encode();
   if (!fn) return false;
-  const cuuint64_t pitch = (cuuint64_t)9 * P * kKB;
-  const cuuint64_t dim[5] = {kKB, (cuuint64_t)rows, (cuuint64_t)P, 9, (cuuint64_t)units};
-  const cuuint64_t str[4] = {pitch, kKB, (cuuint64_t)P * kKB, pitch * rows};
-  const cuuint32_t bx[5] = {kKB, (cuuint32_t)box, (cuuint32_t)P, 1, 1}, one[5] = {1, 1, 1, 1, 1};
-  return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, base, dim, str, bx, one,
+  const cuuint64_t all = (cuuint64_t)kRow * rows;
+  const cuuint32_t one[5] = {1, 1, 1, 1, 1};
+  const cuuint64_t dim2[5] = {2 * kKB, (cuuint64_t)rows, 3, 9, (cuuint64_t)units};
+  const cuuint64_t str2[4] = {kRow, 2 * kKB, 6 * kKB, all};
+  const cuuint32_t box2[5] = {2 * kKB, (cuuint32_t)box, 3, 1, 1};
+  const cuuint64_t dim1[4] = {kKB, (cuuint64_t)rows, 9, (cuuint64_t)units};
+  const cuuint64_t str1[3] = {kRow, kKB, all};
+  const cuuint32_t box1[4] = {kKB, (cuuint32_t)box, 1, 1};
+  return fn(pairs, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, base, dim2, str2, box2, one,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS &&
+         fn(single, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, base + kSingle, dim1, str1, box1, one,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace
+
+static void* slice_kernel(int TN) {
+  switch (TN) {
+    case 16: return (void*)k_slice_gram<16>;
+    case 32: return (void*)k_slice_gram<32>;
+    case 48: return (void*)k_slice_gram<48>;
+    default: return (void*)k_slice_gram<64>;
+  }
+}
 
 bool slice_plan(SlicePlan& p, const Geo& g, int bc, int msl, int mwlt, int mwlr,
                 size_t budget) {
@@ -599,16 +657,15 @@ bool slice_plan(SlicePlan& p, const Geo& g, int bc, int msl, int mwlt, int mwlr,
   while (p.tmem_cols < kPlanes * p.TN) p.tmem_cols *= 2;
   // column units per chunk: as many as the budget holds, in equal chunks
   const int units = 3 * p.ntile;
-  const size_t unit = (size_t)mwlr * 9 * kPlanes * kKB * (p.rows_a + p.rows_b);
+  const size_t unit = (size_t)mwlr * kRow * (p.rows_a + p.rows_b);
   long long nuc = (long long)(budget / unit);
   if (nuc < 1) return false;
   if (nuc > units) nuc = units;
   p.nchunk = (int)((units + nuc - 1) / nuc);
   p.nuc = (units + p.nchunk - 1) / p.nchunk;
   p.nchunk = (units + p.nuc - 1) / p.nuc;
-  const size_t kb = (size_t)mwlr * p.nuc * 9;
-  p.bytes_a = kb * kPlanes * p.rows_a * kKB;
-  p.bytes_b = kb * kPlanes * p.rows_b * kKB;
+  p.bytes_a = (size_t)mwlr * p.nuc * p.rows_a * kRow;
+  p.bytes_b = (size_t)mwlr * p.nuc * p.rows_b * kRow;
   p.nwl = (size_t)msl * msl * mwlt * mwlr * p.N0;
   p.acc_bytes = p.nwl * 2 * sizeof(unsigned long long);
   // column splits: enough for the 32-bit range, then the fewest waves of the
@@ -634,8 +691,8 @@ bool slice_in_range(double dev, double delta, int mwlr) {
   return std::pow(1.0 + 3.0 * delta, 0.5 * mwlr) / (1.0 - 3.0 * dev) <= 1.98;
 }
 
-int slice_prepare() {
-  void* fn = (void*)k_slice_gram;
+int slice_prepare(const SlicePlan& p) {
+  void* fn = slice_kernel(p.TN);
   static std::mutex mu;
   static std::set<std::pair<int, void*>> done;
   int dev = 0;
@@ -689,9 +746,10 @@ void slice_lines(const Geo& g, const SlicePlan& p, int chunk, const double* uh,
 
 void slice_gram(const SlicePlan& p, int chunk, unsigned char* sa, unsigned char* sb,
                 unsigned long long* acc, int* fail, cudaStream_t st) {
-  CUtensorMap ma, mb;
+  CUtensorMap ma2, ma1, mb2, mb1;
   const long long un = (long long)p.mwlr * p.nuc;
-  if (!plane_map(&ma, sa, p.rows_a, un, 128) || !plane_map(&mb, sb, p.rows_b, un, p.TN)) {
+  if (!plane_maps(&ma2, &ma1, sa, p.rows_a, un, 128) ||
+      !plane_maps(&mb2, &mb1, sb, p.rows_b, un, p.TN)) {
     set_error("kernel slice_gram: tensor map refused");
     return;
   }
@@ -717,8 +775,8 @@ void slice_gram(const SlicePlan& p, int chunk, unsigned char* sa, unsigned char*
   a.fail = fail;
   const long long items = (long long)p.mwlr * p.nsplit * p.ntiles;
   const unsigned grid = (unsigned)std::min<long long>(items, num_sms());
-  void* args[] = {&ma, &mb, &a};
-  cudaLaunchKernel((void*)k_slice_gram, dim3(grid), dim3(kGramThreads), args, p.smem, st);
+  void* args[] = {&ma2, &ma1, &mb2, &mb1, &a};
+  cudaLaunchKernel(slice_kernel(p.TN), dim3(grid), dim3(kGramThreads), args, p.smem, st);
   WLG_LAUNCH_CHECK("slice_gram");
 }
 

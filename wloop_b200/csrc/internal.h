@@ -208,7 +208,7 @@ bool slice_plan(SlicePlan& p, const Geo& g, int bc, int msl, int mwlt, int mwlr,
 // and max |U^dag U - 1| over the levels (false for NaN)
 bool slice_in_range(double dev, double delta, int mwlr);
 // shared-memory limit and driver entry point (before any launch or capture)
-int slice_prepare();
+int slice_prepare(const SlicePlan& p);
 // *dev (device): max |U^dag U - 1| over the msl levels, as double bits
 void levels_deviation(const Geo& g, int msl, const double2* levels,
                       unsigned long long* dev, cudaStream_t st);
