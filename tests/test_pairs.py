@@ -98,3 +98,22 @@ def test_same_bits(case):
         ref = c.measure(p)
         assert c.contract_form == 11 and c.kernel_time("contract")[1] == r
     assert np.isfinite(ref).all() and np.array_equal(got, ref)
+
+
+@pytest.mark.gpu
+def test_same_bits_every_time():
+    """Blocks of three warps, two per SM, three stages, several passes: the case
+    in which a warp once freed a stage before its last read of it."""
+    n, p = (48, 24, 24, 24), WloopParms(msl=4, nss=[0, 1, 1, 1], mwlt=12, mwlr=12, op_smear=APE,
+                                        alpha_ape=0.5, proj_iter=4)
+    shape = plan(n, 3, 4, 12, 12)
+    assert shape["block"] == 96 and shape["ctas"] == 2 and shape["npass"] > 1
+    with Context(n, 3, "mixed") as c:
+        c.generate(5, 0.2)
+        c.snapshot()
+        c.set_gram_tuning(stages=2)
+        ref = c.measure(p)
+        c.set_gram_tuning()
+        for _ in range(12):
+            c.restore()
+            assert np.array_equal(c.measure(p), ref)

@@ -284,6 +284,9 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
           }
         }
+        // every lane's reads of the slot are done before lane 0 frees it (its
+        // arrive alone does not keep the last read of the other lanes ahead)
+        __threadfence_block();
         __syncwarp();
         if (lane == 0) mbar_arrive(empty + s);
         if (++s == p.stages) {
