@@ -592,7 +592,7 @@ template <class T> int issue(wlg_batch* b, int phase) {
         gauge_chain<T>(f.g, f.gp, lview<T>(b->arena + f.U, f.D, 4, 0).p[0],
                        (double*)(b->arena + f.gG), (double*)(b->arena + f.gH),
                        (unsigned long long*)(b->arena + f.gDev), b->st);
-        kernels++;
+        kernels += 2;
         if (f.slices) {
           levels_deviation(f.g, f.p.msl,
                            (const double2*)(b->arena + f.region + 6 * f.D * elem_bytes(b)),

@@ -55,11 +55,6 @@
 namespace wlg {
 namespace {
 
-__device__ __forceinline__ void unit(M3<double>& m) {
-  zero(m);
-  m.e[0].x = m.e[4].x = m.e[8].x = 1.0;
-}
-
 // 3x3 complex inverse by cofactors, inv = adj(h) / det(h)
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -98,50 +93,87 @@ __device__ __forceinline__ void inverse3(M3<double>& inv, const M3<double>& h) {
 }
 
 // ---------------------------------------------------------------------------
-// g(y0, j) and H^-1(y0, j) = (g g^dag)^-1 for y0 in [0, Nu): g(0) = 1,
-// g(y0+1) = g(y0) U0(y0 mod N0, j); FP64 slabs.  One thread per spatial site
-// (the chain is sequential in time).  *dev receives max |H - 1| over the
-// sites (as the bits of a non-negative double, atomicMax).
+// g(y0, j) for y0 in [0, Nu): g(0) = 1, g(y0+1) = g(y0) U0(y0 mod N0, j); FP64
+// slab.  The chain is sequential in time, but the rows of g are independent:
+// one thread per spatial site and row (the three rows of a 32-site tile in
+// neighbouring warps, which share U0 through L1), the next link loaded before
+// the current product.  The gauge stage of a 32x16^3 lattice (4096 chains): 0.18
+// ms, 0.21 with one thread per site, the inverse below in the chain and no link
+// ahead.
 // ---------------------------------------------------------------------------
 template <class T>
-__global__ void __launch_bounds__(128) k_gauge_chain(Geo g, int Nu, int ntile,
-                                                     const typename V2<T>::t* __restrict__ u0,
-                                                     double* __restrict__ G,
-                                                     double* __restrict__ Hinv,
-                                                     unsigned long long* __restrict__ dev) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  double worst = 0.0;
-  if (j < ntile * 32) {
-    const int jt = j >> 5, lane = j & 31;
-    if (j >= g.vs) {
-      for (int y0 = 0; y0 < Nu; y0++) {
-        zero_slab(G, slab_tile(y0, ntile, jt), lane);
-        zero_slab(Hinv, slab_tile(y0, ntile, jt), lane);
-      }
-    } else {
-      M3<double> m, t, ud;
-      unit(m);
-      for (int y0 = 0; y0 < Nu; y0++) {
-        const size_t tile = slab_tile(y0, ntile, jt);
-        st_slab(G, tile, lane, m);
-        mul_ad(t, m, m);  // H = g g^dag
+__global__ void __launch_bounds__(96) k_gauge_chain(Geo g, int Nu, int ntile,
+                                                    const typename V2<T>::t* __restrict__ u0,
+                                                    double* __restrict__ G) {
+  const int jt = blockIdx.x, row = threadIdx.x >> 5, lane = threadIdx.x & 31, j = jt * 32 + lane;
+  double* out = G + (size_t)jt * kSlabTile + row * 6 * 32 + lane;
+  const size_t step = (size_t)ntile * kSlabTile;
+  const bool live = j < g.vs;
+  const int at = live ? j : g.vs - 1;
+  double2 m[3];
 #pragma unroll
-        for (int e = 0; e < 9; e++) {
-          const double dr = fabs(t.e[e].x - ((e % 4 == 0) ? 1.0 : 0.0)), di = fabs(t.e[e].y);
-          if (!(dr <= worst)) worst = dr;  // a NaN sticks
-          if (!(di <= worst)) worst = di;
-        }
-        inverse3(ud, t);
-        st_slab(Hinv, tile, lane, ud);
-        if (y0 + 1 < Nu) {
-          M3<T> u;
-          ld<T>(u, u0, g.vol, (y0 % g.n[0]) * g.vs + j);
-          cvt(ud, u);
-          mul(t, m, ud);
-          m = t;
-        }
-      }
+  for (int k = 0; k < 3; k++) m[k] = make_double2(live && k == row ? 1.0 : 0.0, 0.0);
+  M3<T> u, next;
+  ld<T>(next, u0, g.vol, at);
+  int x0 = 0;
+  for (int y0 = 0; y0 < Nu; y0++) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      out[(2 * k) * 32] = m[k].x;
+      out[(2 * k + 1) * 32] = m[k].y;
     }
+    out += step;
+    if (y0 + 1 == Nu) break;
+    u = next;
+    if (++x0 == g.n[0]) x0 = 0;
+    if (y0 + 2 < Nu) ld<T>(next, u0, g.vol, x0 * g.vs + at);
+    M3<double> ud;
+    cvt(ud, u);
+    double2 t[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {  // row `row` of mul()
+      double re = m[0].x * ud.e[c].x - m[0].y * ud.e[c].y;
+      double im = m[0].x * ud.e[c].y + m[0].y * ud.e[c].x;
+#pragma unroll
+      for (int k = 1; k < 3; k++) {
+        re = fma(m[k].x, ud.e[3 * k + c].x, re);
+        re = fma(-m[k].y, ud.e[3 * k + c].y, re);
+        im = fma(m[k].x, ud.e[3 * k + c].y, im);
+        im = fma(m[k].y, ud.e[3 * k + c].x, im);
+      }
+      t[c] = make_double2(re, im);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) m[k] = t[k];
+  }
+}
+
+// H^-1 = (g g^dag)^-1 of every site; *dev receives max |H - 1| over the sites
+// (as the bits of a non-negative double, atomicMax)
+__global__ void __launch_bounds__(128) k_gauge_inverse(long long nlane, int vs, int ntile,
+                                                       const double* __restrict__ G,
+                                                       double* __restrict__ Hinv,
+                                                       unsigned long long* __restrict__ dev) {
+  double worst = 0.0;
+  for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < nlane;
+       w += (long long)gridDim.x * blockDim.x) {
+    const size_t tile = (size_t)(w >> 5);
+    const int lane = (int)(w & 31);
+    if ((int)(tile % ntile) * 32 + lane >= vs) {
+      zero_slab(Hinv, tile, lane);
+      continue;
+    }
+    M3<double> m, t, h;
+    ld_slab(m, G, tile, lane);
+    mul_ad(t, m, m);  // H = g g^dag
+#pragma unroll
+    for (int e = 0; e < 9; e++) {
+      const double dr = fabs(t.e[e].x - ((e % 4 == 0) ? 1.0 : 0.0)), di = fabs(t.e[e].y);
+      if (!(dr <= worst)) worst = dr;  // a NaN sticks
+      if (!(di <= worst)) worst = di;
+    }
+    inverse3(h, t);
+    st_slab(Hinv, tile, lane, h);
   }
   // NaN (a singular chain) compares as the largest value
   if (worst != worst) worst = 1e300;
@@ -648,10 +680,13 @@ bool gram_plan(GramPlan& p, const Geo& g, int bc, int msl, int mwlt, bool fp64,
 template <class T>
 void gauge_chain(const Geo& g, const GramPlan& p, const typename V2<T>::t* u0, double* G,
                  double* Hinv, unsigned long long* dev, cudaStream_t st) {
-  const int nthr = p.ntile * 32;
   cudaMemsetAsync(dev, 0, sizeof(unsigned long long), st);
-  k_gauge_chain<T><<<(nthr + 127) / 128, 128, 0, st>>>(g, p.Nu, p.ntile, u0, G, Hinv, dev);
+  k_gauge_chain<T><<<p.ntile, 96, 0, st>>>(g, p.Nu, p.ntile, u0, G);
   WLG_LAUNCH_CHECK("gauge_chain");
+  const long long n = (long long)p.Nu * p.ntile * 32;
+  const long long grid = std::min<long long>((n + 127) / 128, num_sms() * 16);
+  k_gauge_inverse<<<(int)grid, 128, 0, st>>>(n, g.vs, p.ntile, G, Hinv, dev);
+  WLG_LAUNCH_CHECK("gauge_inverse");
 }
 
 template <class T>
