@@ -65,7 +65,7 @@ struct wlg_ctx {
   Geo g;
   cudaStream_t st = nullptr;
   DevBuf U, U0, bar, til, apeA, apeB, dl, levels, lines, lines2, partial, wl, plaq_part, plaq_out,
-      staging, ipt;
+      plaq_count, staging, ipt;
   // the temporal-gauge form: g, H^-1, recursion links, B and A lines, the
   // unitarity deviation of g
   DevBuf gG, gH, gUh, gB, gA, gDev;
@@ -304,8 +304,12 @@ template <class T> static int do_hyp_spatial(wlg_ctx* c, double a1, double a2, i
 
 template <class T> static int do_plaq(wlg_ctx* c, Links<T> L, double* dev_out) {
   if (ensure(c->plaq_part, sizeof(double) * plaq_partials())) return -1;
+  if (!c->plaq_count.p) {
+    if (ensure(c->plaq_count, sizeof(unsigned))) return -1;
+    WLG_CUDA(cudaMemsetAsync(c->plaq_count.p, 0, sizeof(unsigned), c->st));
+  }
   ProfScope ps(c, "plaq");
-  plaq_sum<T>(c->g, c->bc, L, (double*)c->plaq_part.p, dev_out, c->st);
+  plaq_sum<T>(c->g, c->bc, L, (double*)c->plaq_part.p, (unsigned*)c->plaq_count.p, dev_out, c->st);
   return 0;
 }
 
@@ -833,7 +837,7 @@ int wlg_destroy(wlg_ctx* c) {
   if (c->cst) cudaStreamSynchronize(c->cst);
   harvest(c);
   DevBuf* all[] = {&c->U, &c->U0, &c->bar, &c->til, &c->apeA, &c->apeB, &c->dl, &c->levels, &c->lines, &c->lines2,
-                   &c->gG, &c->gH, &c->gUh, &c->gB, &c->gA, &c->gDev, &c->gSa, &c->gSb, &c->gAcc, &c->partial, &c->wl, &c->plaq_part, &c->plaq_out, &c->staging, &c->ipt,
+                   &c->gG, &c->gH, &c->gUh, &c->gB, &c->gA, &c->gDev, &c->gSa, &c->gSb, &c->gAcc, &c->partial, &c->wl, &c->plaq_part, &c->plaq_out, &c->plaq_count, &c->staging, &c->ipt,
                    &c->prefetch_buf};
   for (DevBuf* b : all) release(*b);
   for (cudaEvent_t e : c->evpool) cudaEventDestroy(e);

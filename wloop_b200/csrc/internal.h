@@ -67,9 +67,10 @@ void staples_lnks(int n, const double* u1, const double* u2, const double* u3, d
 // In-place projection of n packed FP64 matrices (18 doubles each).
 void project_batch(double* m, int n, int iter, cudaStream_t st);
 // Plaquette sum (lnkplaq.c:48-128) into *out (device double); partial holds
-// at least plaq_partials() doubles.
+// at least plaq_partials() doubles; *count (device) is zero before and after.
 template <class T>
-void plaq_sum(const Geo& g, int bc, Links<T> U, double* partial, double* out, cudaStream_t st);
+void plaq_sum(const Geo& g, int bc, Links<T> U, double* partial, unsigned* count, double* out,
+              cudaStream_t st);
 int plaq_partials();
 // FP64 plaquette sum of a field in device memory in the AoS lexicographic
 // su3_dble layout of the host (noalloc.cu); partials must hold
@@ -159,6 +160,7 @@ constexpr long long kGramMinSites = 32768;
 // The gauge field g and H^-1 = (g g^dag)^-1 (FP64 slabs of A doubles each)
 // from the temporal links u0; *dev (device) receives max |g g^dag - 1| as the
 // bits of a non-negative double (the form is not used when it exceeds 1/4).
+// Two launches.
 template <class T>
 void gauge_chain(const Geo& g, const GramPlan& p, const typename V2<T>::t* u0, double* G,
                  double* Hinv, unsigned long long* dev, cudaStream_t st);
@@ -305,6 +307,34 @@ void shift_links(const Geo& g, Links<T> src, Links<T> dst, const int s[4], cudaS
 // Writes the synthetic link field of the given seed/eps straight into SoA.
 template <class T>
 void generate_soa(const Geo& g, int bc, uint64_t seed, double eps, Links<T> U, cudaStream_t st);
+
+// ---- launches that overlap the kernel before them ----------------------------
+// A kernel launched by launch_after may be set up while its predecessor on the
+// stream still runs; it must pass its work index through after_previous before
+// it touches memory (the wait for the predecessor's end; the index makes every
+// later access depend on it).  Used where a chain of short kernels would
+// otherwise spend a launch latency between each two.
+#ifdef __CUDACC__
+__device__ __forceinline__ long long after_previous(long long w) {
+  asm volatile("griddepcontrol.launch_dependents;\n griddepcontrol.wait;\n" : "+l"(w)::"memory");
+  return w;
+}
+template <class... P, class... Q>
+inline void launch_after(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st,
+                         Q... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+#endif
 
 // ---- error handling and launch accounting ---------------------------------
 void set_error(const char* fmt, ...);

@@ -761,7 +761,7 @@ __device__ __forceinline__ void contract4_body(const CArgs<T>& A, int bid) {
 
 template <class T, int G, int MSL, int MINB, bool BULK, int PK>
 __global__ void __launch_bounds__(128, MINB) k_contract4(CArgs<T> A) {
-  contract4_body<T, G, MSL, BULK, PK>(A, blockIdx.x);
+  contract4_body<T, G, MSL, BULK, PK>(A, (int)after_previous(blockIdx.x));
 }
 
 template <class T, int G, int MSL, int MINB, bool BULK, int PK>
@@ -1004,7 +1004,7 @@ static void launch_contract4_m(const Geo& g, const ContractPlan& p, const typena
   A.partial = partial;
   A.level = level;
   A.next = next;
-  kern<<<g.n[0] * p.ngrp * p.nCB, p.block, smem, st>>>(A);
+  launch_after(kern, g.n[0] * p.ngrp * p.nCB, p.block, smem, st, A);
   WLG_LAUNCH_CHECK("contract");
 }
 
@@ -1163,7 +1163,8 @@ __device__ __forceinline__ void reduce_item(const RArgs& A, int i) {
 }
 
 __global__ void k_contract_reduce(RArgs A, int nout) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nout; i += gridDim.x * blockDim.x)
+  for (int i = (int)after_previous(blockIdx.x * blockDim.x + threadIdx.x); i < nout;
+       i += gridDim.x * blockDim.x)
     reduce_item(A, i);
 }
 
@@ -1197,7 +1198,7 @@ void contract_reduce(const Geo& g, const ContractPlan& p, int msl, int mwlt, int
                      const double* partial, double* wl_mat, cudaStream_t st) {
   RArgs A = reduce_args(g, p, msl, mwlt, mwlr, r, partial, wl_mat);
   int grid = (A.nout + 255) / 256;
-  k_contract_reduce<<<grid, 256, 0, st>>>(A, A.nout);
+  launch_after(k_contract_reduce, grid, 256, 0, st, A, A.nout);
   WLG_LAUNCH_CHECK("contract_reduce");
 }
 

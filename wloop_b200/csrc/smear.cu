@@ -10,6 +10,8 @@
 // always run in FP64.
 #include <string.h>
 
+#include <algorithm>
+
 #include "internal.h"
 
 namespace wlg {
@@ -215,8 +217,8 @@ template <class T> __device__ __forceinline__ void hyp3_l2_item(const SArgs<T>& 
   st(A.D.p[mu], g.vol, s, o);
 }
 
-#define WLG_GRID_STRIDE(n) \
-  for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < (n); \
+#define WLG_GRID_STRIDE(n)                                                                     \
+  for (long long w = after_previous(blockIdx.x * (long long)blockDim.x + threadIdx.x); w < (n); \
        w += (long long)gridDim.x * blockDim.x)
 
 // batched: one grid over the flattened work of n lattices
@@ -292,8 +294,8 @@ __global__ void k_project_batch(double* m, int n, int iter) {
 // products in T, sums in FP64; warp shuffle + block reduction into one
 // partial per block, then a fixed-order final pass (deterministic).
 // ---------------------------------------------------------------------------
-constexpr int kPlaqBlocks = 1184;  // 8 x 148 SMs
-constexpr int kPlaqThreads = 256;
+constexpr int kPlaqBlocks = 1776;  // 12 x 148 SMs
+constexpr int kPlaqThreads = 192;  // six planes of a tile
 int plaq_partials() { return kPlaqBlocks; }
 
 template <class T>
@@ -326,27 +328,51 @@ __device__ __forceinline__ double block_sum(double v) {
   return r;
 }
 
-template <class T>
-__global__ void __launch_bounds__(kPlaqThreads) k_plaq(Geo g, int bc, Links<T> U, double* partial) {
-  double acc = 0.0;
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < g.vol; s += gridDim.x * blockDim.x) {
-    int x[4];
-    coords(g, s, x);
-    double pa = 0.0;
-    for (int mu = 1; mu < 4; mu++) {
-      if (x[0] < g.n[0] - 1 || bc != 0) pa += plaq_at(g, U, x, s, mu, 0);
-      for (int nu = 1; nu < mu; nu++) pa += plaq_at(g, U, x, s, mu, nu);
+// PLANES: one thread per (site, plane), the six planes of a 32-site tile in
+// neighbouring warps, for lattices whose sites alone leave most of the GPU's
+// warps empty (8^4: 10.4 us a call, 17.3 with one thread per site and a second
+// kernel for the blocks' sums); otherwise one thread per site and its planes
+// in turn (64x32^3 mixed 249 us, 271 with PLANES).  The block that finishes
+// last adds the blocks' sums, in order; *count returns to zero.
+template <class T, bool PLANES>
+__global__ void __launch_bounds__(kPlaqThreads) k_plaq(Geo g, int bc, Links<T> U, double* partial,
+                                                       unsigned* count, double* out) {
+  __shared__ bool last;
+  double sum = 0.0;
+  const long long n = PLANES ? tile_items(g.vol, 6) : g.vol;
+  for (long long w = after_previous(blockIdx.x * (long long)blockDim.x + threadIdx.x); w < n;
+       w += (long long)gridDim.x * blockDim.x) {
+    int x[4], q = 0, s = (int)w;
+    if (PLANES) {
+      tile_item(w, 6, q, s);
+      if (s >= g.vol) continue;
     }
-    acc += pa;
+    coords(g, s, x);
+    const bool time = bc != 0 || x[0] < g.n[0] - 1;
+    if (PLANES) {  // (1,0) (2,0) (2,1) (3,0) (3,1) (3,2)
+      const int mu = q == 0 ? 1 : (q < 3 ? 2 : 3), nu = q == 0 ? 0 : (q < 3 ? q - 1 : q - 3);
+      if (nu > 0 || time) sum += plaq_at(g, U, x, s, mu, nu);
+    } else {
+      double pa = 0.0;
+      for (int mu = 1; mu < 4; mu++) {
+        if (time) pa += plaq_at(g, U, x, s, mu, 0);
+        for (int nu = 1; nu < mu; nu++) pa += plaq_at(g, U, x, s, mu, nu);
+      }
+      sum += pa;
+    }
   }
-  double r = block_sum(acc);
-  if (threadIdx.x == 0) partial[blockIdx.x] = r;
-}
-
-__global__ void k_sum_partials(const double* partial, int n, double* out) {
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) acc += partial[i];
-  double r = block_sum(acc);
+  double r = block_sum(sum);
+  if (threadIdx.x == 0) {
+    partial[blockIdx.x] = r;
+    __threadfence();
+    last = atomicInc(count, gridDim.x - 1) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  sum = 0.0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) sum += __ldcg(partial + i);
+  r = block_sum(sum);
   if (threadIdx.x == 0) *out = r;
 }
 
@@ -425,7 +451,7 @@ void hyp_level3(const Geo& g, Links<T> U, typename V2<T>::t* vbar, double a3, in
   A.b = a3 / 2.0;
   A.proj = proj;
   A.iter = iter;
-  k_hyp_l3<T><<<grid_for(tile_items(g.vol, 12), 128), 128, 0, st>>>(A);
+  launch_after(k_hyp_l3<T>, grid_for(tile_items(g.vol, 12), 128), 128, 0, st, A);
   WLG_LAUNCH_CHECK("hyp_level3");
 }
 template <class T>
@@ -439,7 +465,7 @@ void hyp_level2(const Geo& g, Links<T> U, const typename V2<T>::t* vbar, typenam
   A.b = a2 / 4.0;
   A.proj = proj;
   A.iter = iter;
-  k_hyp_l2<T><<<grid_for(tile_items(g.vol, 12), 128), 128, 0, st>>>(A);
+  launch_after(k_hyp_l2<T>, grid_for(tile_items(g.vol, 12), 128), 128, 0, st, A);
   WLG_LAUNCH_CHECK("hyp_level2");
 }
 template <class T>
@@ -457,7 +483,7 @@ void hyp_level1(const Geo& g, Links<T> U, const typename V2<T>::t* vtil, double 
   A.mu0 = mu0;
   A.nmu = nmu;
   A.bc = bc;
-  k_hyp_l1<T><<<grid_for(tile_items(g.vol, nmu), 128), 128, 0, st>>>(A);
+  launch_after(k_hyp_l1<T>, grid_for(tile_items(g.vol, nmu), 128), 128, 0, st, A);
   WLG_LAUNCH_CHECK("hyp_level1");
 }
 template <class T>
@@ -470,7 +496,7 @@ void ape_sweep(const Geo& g, Links<T> src, Links<T> dst, double alpha, int proj,
   A.proj = proj;
   A.iter = iter;
   A.mu0 = mu0;
-  k_ape<T><<<grid_for(ape_items(g.vol, mu0), 128), 128, 0, st>>>(A);
+  launch_after(k_ape<T>, grid_for(ape_items(g.vol, mu0), 128), 128, 0, st, A);
   WLG_LAUNCH_CHECK("ape_sweep");
 }
 template <class T>
@@ -483,7 +509,7 @@ void hyp3d_level1(const Geo& g, Links<T> U, typename V2<T>::t* dl, double a2, in
   A.b = a2 / 2.0;
   A.proj = proj;
   A.iter = iter;
-  k_hyp3_l1<T><<<grid_for(6LL * g.vol, 128), 128, 0, st>>>(A);
+  launch_after(k_hyp3_l1<T>, grid_for(6LL * g.vol, 128), 128, 0, st, A);
   WLG_LAUNCH_CHECK("hyp3d_level1");
 }
 template <class T>
@@ -496,7 +522,7 @@ void hyp3d_level2(const Geo& g, Links<T> U, const typename V2<T>::t* dl, double 
   A.b = a1 / 4.0;
   A.proj = proj;
   A.iter = iter;
-  k_hyp3_l2<T><<<grid_for(3LL * g.vol, 128), 128, 0, st>>>(A);
+  launch_after(k_hyp3_l2<T>, grid_for(3LL * g.vol, 128), 128, 0, st, A);
   WLG_LAUNCH_CHECK("hyp3d_level2");
 }
 template <class T>
@@ -528,11 +554,16 @@ void project_batch(double* m, int n, int iter, cudaStream_t st) {
   WLG_LAUNCH_CHECK("project_batch");
 }
 template <class T>
-void plaq_sum(const Geo& g, int bc, Links<T> U, double* partial, double* out, cudaStream_t st) {
-  k_plaq<T><<<kPlaqBlocks, kPlaqThreads, 0, st>>>(g, bc, U, partial);
+void plaq_sum(const Geo& g, int bc, Links<T> U, double* partial, unsigned* count, double* out,
+              cudaStream_t st) {
+  const bool planes = (long long)g.vol < (long long)num_sms() * 512;
+  const long long n = planes ? tile_items(g.vol, 6) : g.vol;
+  const int grid = (int)std::min<long long>((n + kPlaqThreads - 1) / kPlaqThreads, kPlaqBlocks);
+  if (planes)
+    launch_after(k_plaq<T, true>, grid, kPlaqThreads, 0, st, g, bc, U, partial, count, out);
+  else
+    launch_after(k_plaq<T, false>, grid, kPlaqThreads, 0, st, g, bc, U, partial, count, out);
   WLG_LAUNCH_CHECK("plaq_sum");
-  k_sum_partials<<<1, 1024, 0, st>>>(partial, kPlaqBlocks, out);
-  WLG_LAUNCH_CHECK("plaq_sum_final");
 }
 
 #define WLG_INST(T)                                                                               \
@@ -546,7 +577,7 @@ void plaq_sum(const Geo& g, int bc, Links<T> U, double* partial, double* out, cu
   template void hyp3d_level2<T>(const Geo&, Links<T>, const V2<T>::t*, double, int, int,          \
                                 cudaStream_t);                                                    \
   template void staple_sum<T>(const Geo&, Links<T>, Links<T>, int, int, Links<T>, cudaStream_t);  \
-  template void plaq_sum<T>(const Geo&, int, Links<T>, double*, double*, cudaStream_t);    \
+  template void plaq_sum<T>(const Geo&, int, Links<T>, double*, unsigned*, double*, cudaStream_t); \
   template void smear_batch<T>(int, const SArgs<T>*, const long long*, int, long long, cudaStream_t);
 
 WLG_INST(double)
