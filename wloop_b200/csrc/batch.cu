@@ -349,13 +349,13 @@ template <class T> void build_ops(wlg_batch* b, int phase) {
           ape.push_back(x);
           u3.push_back(ape_items(f.g.vol, 1));
         } else {
-          // spatial HYP: level 1 from cur into dl, copy cur -> dst, level 2 in place on dst
+          // spatial HYP: level 1 from cur into dl, level 2 from cur and dl into dst
           x.U = cur[c];
           x.aux0 = (T2*)dl[c];
           x.a = 1.0 - f.p.alpha_hyp[1];
           x.b = f.p.alpha_hyp[1] / 2.0;
           h1.push_back(x);
-          u6.push_back(6LL * f.g.vol);
+          u6.push_back(tile_items(f.g.vol, 6));
           x.D = dst;
           x.a = 1.0 - f.p.alpha_hyp[0];
           x.b = f.p.alpha_hyp[0] / 4.0;
@@ -367,14 +367,7 @@ template <class T> void build_ops(wlg_batch* b, int phase) {
       if (!h1.empty()) {
         push_smear(BATCH_HYP3D1, h1, u6);
         std::vector<long long> u3h;
-        for (auto& x : h2) {
-          u3h.push_back(3LL * x.g.vol);
-          // the source of this sweep is h1's U for the same lattice
-        }
-        for (size_t j = 0; j < h2.size(); j++)
-          for (int k = 1; k < 4; k++)
-            if (h1[j].U.p[k] != h2[j].D.p[k])
-              push_copy(h2[j].D.p[k], h1[j].U.p[k], link_elems<T>(h2[j].g.vol) * elem_bytes(b));
+        for (auto& x : h2) u3h.push_back(tile_items(x.g.vol, 3));
         push_smear(BATCH_HYP3D2, h2, u3h);
       }
     }

@@ -277,13 +277,7 @@ template <class T> static int hyp3_sweep(wlg_ctx* c, Links<T> src, Links<T> dst,
                                          double a2, int proj, int piter) {
   if (ensure(c->dl, field_bytes(c, 6))) return -1;
   hyp3d_level1<T>(c->g, src, (typename V2<T>::t*)c->dl.p, a2, proj, piter, c->st);
-  if (src.p[1] != dst.p[1]) {
-    // level 2 reads only its own src link for the linear combination
-    for (int k = 1; k < 4; k++)
-      WLG_CUDA(cudaMemcpyAsync(dst.p[k], src.p[k], dir_bytes(c),
-                               cudaMemcpyDeviceToDevice, c->st));
-  }
-  hyp3d_level2<T>(c->g, dst, (const typename V2<T>::t*)c->dl.p, a1, proj, piter, c->st);
+  hyp3d_level2<T>(c->g, src, dst, (const typename V2<T>::t*)c->dl.p, a1, proj, piter, c->st);
   return 0;
 }
 

@@ -49,13 +49,13 @@ template <class T>
 void ape_sweep(const Geo& g, Links<T> src, Links<T> dst, double alpha, int proj, int iter,
                int mu0, cudaStream_t st);
 // Two-level spatial HYP (hyp_spatial_links.c:160-344); dl holds 2 slots x 3
-// spatial directions; U's spatial links are updated in place.
+// spatial directions; level 2 writes D, which may be U.
 template <class T>
 void hyp3d_level1(const Geo& g, Links<T> U, typename V2<T>::t* dl, double a2, int proj, int iter,
                   cudaStream_t st);
 template <class T>
-void hyp3d_level2(const Geo& g, Links<T> U, const typename V2<T>::t* dl, double a1, int proj,
-                  int iter, cudaStream_t st);
+void hyp3d_level2(const Geo& g, Links<T> U, Links<T> D, const typename V2<T>::t* dl, double a1,
+                  int proj, int iter, cudaStream_t st);
 // staple_sum (staple_sum.c:53-87): vb(x,mu) += staples in the (mu,nu) plane.
 template <class T>
 void staple_sum(const Geo& g, Links<T> u1, Links<T> u2, int mu, int nu, Links<T> vb,

@@ -175,10 +175,14 @@ template <class T> __device__ __forceinline__ void ape_item(const SArgs<T>& A, l
 }
 
 // Spatial HYP, level with alpha2 (decorated_links1, hyp_spatial_links.c:210-265)
-//   dl[slot(mu,eta)](x,mu) = P[(1-a2) U + a2/2 S_eta(U)];  w in [0, 6V)
+//   dl[slot(mu,eta)](x,mu) = P[(1-a2) U + a2/2 S_eta(U)];  w in [0, tile_items(V, 6)),
+// tile-major as the APE sweep (a sweep of the two levels at 24^3x48 819 us FP64, 574
+// mixed; 883 and 595 with one output slot after the other over the lattice)
 template <class T> __device__ __forceinline__ void hyp3_l1_item(const SArgs<T>& A, long long w) {
   const Geo& g = A.g;
-  int q = (int)(w / g.vol), s = (int)(w - (long long)q * g.vol);
+  int q, s;
+  tile_item(w, 6, q, s);
+  if (s >= g.vol) return;
   int mu = 1 + q / 2, eta = ((mu + q % 2) % 3) + 1;
   int x[4];
   coords(g, s, x);
@@ -194,10 +198,12 @@ template <class T> __device__ __forceinline__ void hyp3_l1_item(const SArgs<T>& 
 }
 
 // Spatial HYP, level with alpha1 (decorated_links2, hyp_spatial_links.c:160-207),
-// in place on D (lcomb with D's own link);  w in [0, 3V)
+// into D, which may be U (an item reads only its own U link);  w in [0, tile_items(V, 3))
 template <class T> __device__ __forceinline__ void hyp3_l2_item(const SArgs<T>& A, long long w) {
   const Geo& g = A.g;
-  int q = (int)(w / g.vol), s = (int)(w - (long long)q * g.vol);
+  int q, s;
+  tile_item(w, 3, q, s);
+  if (s >= g.vol) return;
   int mu = 1 + q;
   int x[4];
   coords(g, s, x);
@@ -209,7 +215,7 @@ template <class T> __device__ __forceinline__ void hyp3_l2_item(const SArgs<T>& 
     add_staples(S, g, x, s, fld<T>(A.aux0, g.vol, hyp3_slot(nu, mu), nu - 1, 3),
                 fld<T>(A.aux0, g.vol, hyp3_slot(mu, nu), mu - 1, 3), mu, nu);
   }
-  ld(u, A.D.p[mu], g.vol, s);
+  ld(u, A.U.p[mu], g.vol, s);
   M3<double> v;
   lcomb_project(v, A.a, u, A.b, S, A.proj, A.iter);
   M3<T> o;
@@ -256,10 +262,10 @@ __global__ void __launch_bounds__(128, ApeMinBlocks<T>::v) k_ape(SArgs<T> A) {
   WLG_GRID_STRIDE(ape_items(A.g.vol, A.mu0)) ape_item<T>(A, w);
 }
 template <class T> __global__ void __launch_bounds__(128) k_hyp3_l1(SArgs<T> A) {
-  WLG_GRID_STRIDE(6LL * A.g.vol) hyp3_l1_item<T>(A, w);
+  WLG_GRID_STRIDE(tile_items(A.g.vol, 6)) hyp3_l1_item<T>(A, w);
 }
 template <class T> __global__ void __launch_bounds__(128) k_hyp3_l2(SArgs<T> A) {
-  WLG_GRID_STRIDE(3LL * A.g.vol) hyp3_l2_item<T>(A, w);
+  WLG_GRID_STRIDE(tile_items(A.g.vol, 3)) hyp3_l2_item<T>(A, w);
 }
 
 // staple_sum: vb(x,mu) += up + down staples in the (mu,nu) plane
@@ -509,20 +515,21 @@ void hyp3d_level1(const Geo& g, Links<T> U, typename V2<T>::t* dl, double a2, in
   A.b = a2 / 2.0;
   A.proj = proj;
   A.iter = iter;
-  launch_after(k_hyp3_l1<T>, grid_for(6LL * g.vol, 128), 128, 0, st, A);
+  launch_after(k_hyp3_l1<T>, grid_for(tile_items(g.vol, 6), 128), 128, 0, st, A);
   WLG_LAUNCH_CHECK("hyp3d_level1");
 }
 template <class T>
-void hyp3d_level2(const Geo& g, Links<T> U, const typename V2<T>::t* dl, double a1, int proj,
-                  int iter, cudaStream_t st) {
+void hyp3d_level2(const Geo& g, Links<T> U, Links<T> D, const typename V2<T>::t* dl, double a1,
+                  int proj, int iter, cudaStream_t st) {
   SArgs<T> A = sargs<T>(g);
-  A.D = U;
+  A.U = U;
+  A.D = D;
   A.aux0 = const_cast<typename V2<T>::t*>(dl);
   A.a = 1.0 - a1;
   A.b = a1 / 4.0;
   A.proj = proj;
   A.iter = iter;
-  launch_after(k_hyp3_l2<T>, grid_for(3LL * g.vol, 128), 128, 0, st, A);
+  launch_after(k_hyp3_l2<T>, grid_for(tile_items(g.vol, 3), 128), 128, 0, st, A);
   WLG_LAUNCH_CHECK("hyp3d_level2");
 }
 template <class T>
@@ -574,8 +581,8 @@ void plaq_sum(const Geo& g, int bc, Links<T> U, double* partial, unsigned* count
                               int, cudaStream_t);                                                 \
   template void ape_sweep<T>(const Geo&, Links<T>, Links<T>, double, int, int, int, cudaStream_t); \
   template void hyp3d_level1<T>(const Geo&, Links<T>, V2<T>::t*, double, int, int, cudaStream_t); \
-  template void hyp3d_level2<T>(const Geo&, Links<T>, const V2<T>::t*, double, int, int,          \
-                                cudaStream_t);                                                    \
+  template void hyp3d_level2<T>(const Geo&, Links<T>, Links<T>, const V2<T>::t*, double, int,     \
+                                int, cudaStream_t);                                               \
   template void staple_sum<T>(const Geo&, Links<T>, Links<T>, int, int, Links<T>, cudaStream_t);  \
   template void plaq_sum<T>(const Geo&, int, Links<T>, double*, unsigned*, double*, cudaStream_t); \
   template void smear_batch<T>(int, const SArgs<T>*, const long long*, int, long long, cudaStream_t);
