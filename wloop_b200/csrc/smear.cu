@@ -55,7 +55,7 @@ __device__ __forceinline__ void lcomb_project(M3<double>& v, double a, const M3<
     v.e[k].x = a * (double)u.e[k].x + b * (double)s.e[k].x;
     v.e[k].y = a * (double)u.e[k].y + b * (double)s.e[k].y;
   }
-  if (proj) project(v, iter);
+  if (proj) project_as<T>(v, iter);
 }
 
 // ---------------------------------------------------------------------------
@@ -168,7 +168,7 @@ template <class T> __device__ __forceinline__ void ape_item(const SArgs<T>& A, l
     v.e[k].x = (double)u.e[k].x + sr;
     v.e[k].y = (double)u.e[k].y + si;
   }
-  if (A.proj) project(v, A.iter);
+  if (A.proj) project_as<T>(v, A.iter);
   M3<T> o;
   cvt(o, v);
   st(A.D.p[mu], g.vol, s, o);
