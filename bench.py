@@ -371,9 +371,9 @@ class ClockSampler:
                 "reasons": sorted(reasons), "samples": len(sm)}
 
 
-def gram_flops_per_launch(w):
-    """Flops of one banded Gram launch: every (x0, T, s1, s2) is a dot product
-    over 3 directions x vs sites x 18 components."""
+def gram_flops_per_extent(w):
+    """Flops of the banded Gram product of one spatial extent: every (x0, T,
+    s1, s2) is a dot product over 3 directions x vs sites x 18 components."""
     p = w.parms
     vs = w.volume // w.n[0]
     return 2.0 * w.n[0] * p.mwlt * p.msl * p.msl * 3 * vs * 18
@@ -514,9 +514,13 @@ def run_ours(args, rank, world, local):
     # ---- roofline of the dominant kernel (contraction) ----
     c_ms, c_n = kt["contract"]
     per_launch_ms = c_ms / max(1, c_n)
+    # the temporal-gauge form runs all extents of a part of the columns in one
+    # launch: its "launch" below is one extent's share of a measurement
+    digits = form == 11 and args.precision == "fp64" and c_n != kt["hyp"][1] * p.mwlr
     if form == 11:
+        per_launch_ms = c_ms / max(1, kt["hyp"][1] * p.mwlr)
         # the banded Gram product: 2 N0 mwlt msl^2 (3 vs 18) flops per R
-        flops_per_launch = gram_flops_per_launch(w)
+        flops_per_launch = gram_flops_per_extent(w)
     else:
         # the contraction launches also carry the spatial line step of the next R
         flops_per_launch = (fl["contract"] + fl["lines"]) / p.mwlr
@@ -532,6 +536,12 @@ def run_ours(args, rank, world, local):
         peak = max(p_scalar, p_x2)
         peak_src = ("vector FMA probe measured in this run (wlg_peak_flops): the higher of "
                     "scalar fma.rn.f32 and packed fma.rn.f32x2 chains; of measured")
+    if digits:
+        # 28 digit pairs of 8-bit products for each FP64 product
+        flops_per_launch *= 28
+        achieved *= 28
+        peak = 4500.0
+        peak_src = "nominal dense int8 rate (no measured one)"
     traffic = load_traffic().get(args.precision + ("_gram" if form == 11 else ""))
     peaks_file = os.path.join(ROOT, "MEASURED_PEAKS.json")
     hbm, hbm_src = None, None
@@ -552,15 +562,20 @@ def run_ours(args, rank, world, local):
         # its A lines (N0 slices) and B lines (N0 + mwlt slices, periodic), once
         nu = w.n[0] + (p.mwlt if w.bc != 0 else 0)
         bytes_per_launch = link_b * (w.n[0] + nu) * (vol // w.n[0]) * 3 * p.msl
-        kname = "k_gram (banded Gram product of the temporal-gauge lines)"
+        kname = ("k_slice_gram (banded Gram product as exact 8-bit digit products)" if digits else
+                 "k_pair_gram (banded Gram product of the temporal-gauge lines), per extent")
+        if digits:  # 7 digit planes, padded
+            bytes_per_launch = 4096 / 32 * (w.n[0] + nu) * (vol // w.n[0]) * 3 * p.msl
     else:
         bytes_per_launch = link_b * vol * ((3 * p.msl + 1) + 6 * p.msl * (p.mwlr - 1) / p.mwlr)
         kname = "k_contract4 (loop contraction with the fused spatial line step)"
     hbm_ach = bytes_per_launch / (per_launch_ms * 1e-3) / 1e9
     roof = {"kernel": kname, "contract_form": form,
-            "bound": "fp32" if args.precision == "mixed" else "fp64",
-            "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-            "peak_source": peak_src + "; the kernel is bound by CUDA-core FMA throughput, not "
+            "bound": "int8 tensor" if digits else
+                     ("fp32" if args.precision == "mixed" else "fp64"),
+            "achieved": achieved, "peak": peak, "unit": "TOP/s" if digits else "TFLOP/s",
+            "frac": achieved / peak,
+            "peak_source": peak_src if digits else peak_src + "; the kernel is bound by CUDA-core FMA throughput, not "
                            "by HBM (its FP32 dot products need more precision than one "
                            "TF32/BF16 tensor-core pass gives), and MEASURED_PEAKS.json has no "
                            "CUDA-core peak",
