@@ -12,6 +12,7 @@ from tests.test_gpu_parity import assert_wl_close
 from tests.test_gram_plan import LATTICES
 from wloop_b200 import APE, Context, WloopParms, generate_links
 from wloop_b200._native import lib
+from wloop_b200.api import Batch
 
 KEYS = ("rows_a", "rows_b", "tn", "nmt", "ntiles", "stages", "tmem", "smem", "nuc", "nchunk",
         "kps", "nsplit", "bytes_a", "bytes_b", "acc", "ntile")
@@ -106,22 +107,54 @@ def test_loops(case):
     assert np.array_equal(got == 0.0, ref == 0.0)
 
 
+# the spatial links' norm and whether the digits, scaled, hold lines of two links
 @pytest.mark.gpu
-def test_rough_links_leave_the_digits():
-    """Spatial links far from unitary (one projection step short of
-    convergence on a rough field) could leave the digits' range: the FMA
-    kernel measures them."""
+@pytest.mark.parametrize("norm,fits", [(1.2, True), (1.7, True), (3.5, True), (4.3, False)])
+def test_links_far_from_unitary(norm, fits):
+    """Spatial links of norm 1.2 to 4.3 (level 0 is not projected): lines of two of
+    them reach up to norm^2, which the digits hold up to 1.98 x 8 when scaled
+    (exponents 0 to 3); beyond, the FMA kernel measures."""
     n, bc = (8, 4, 4, 4), 3
-    p = WloopParms(msl=2, nss=[0, 2], mwlt=3, mwlr=2, op_smear=1, alpha_hyp=(0.75, 0.6),
-                   proj_iter=3)
-    u = generate_links(n, bc, 77, 0.1)
-    u[:, 1:] *= 1.2  # spatial links of norm 1.2, smeared into level 0 unprojected
+    p = WloopParms(msl=2, nss=[0, 2], mwlt=3, mwlr=2, op_smear=APE, alpha_ape=0.5, proj_iter=3)
+    u = generate_links(n, bc, 77, 0.01)
+    u[:, 1:] *= norm
     with Context(n, bc, "fp64") as c:
         c.set_contract_tuning(variant=11)
         c.upload(u)
         c.set_profiling(True)
         got = c.wloop_sum(p)
         assert c.contract_form == 11
-        assert c.kernel_time("contract")[1] == p.mwlr  # one launch per extent
+        launches = c.kernel_time("contract")[1]
+        c.set_profiling(False)
+        c.upload(u)
+        c.set_gram_tuning(stages=2)
+        fma = c.wloop_sum(p)
+    # one launch per chunk, or one per extent
+    assert launches == (plan(n, bc, 2, 3, 2)["nchunk"] if fits else p.mwlr)
     ref, ref_abs = O.wloop_sum(n, bc, u, p, want_abs=True)
     assert_wl_close(got, ref, ref_abs)
+    columns = 54 * n[1] * n[2] * n[3]
+    assert np.abs(got - fma).max() <= 4.0 * np.sqrt(columns) * 2.0 ** -53 * norm ** 4
+
+
+@pytest.mark.gpu
+def test_spatial_hyp_in_a_batch():
+    """Spatial HYP leaves links far from unitary: a batch scales such a lattice's
+    digits as a context does, with the same bits, also when the next field needs
+    another exponent."""
+    n, bc = (32, 16, 16, 16), 3
+    p = WloopParms(msl=3, nss=[0, 2, 2], mwlt=6, mwlr=5, op_smear=1, alpha_hyp=(0.75, 0.6),
+                   proj_iter=4)
+    fields = [generate_links(n, bc, 91 + k, eps) for k, eps in enumerate((0.2, 0.05, 0.3))]
+    with Context(n, bc, "fp64") as c, Batch([(n, bc, p)], "fp64") as b:
+        for u in fields:
+            c.upload(u)
+            c.set_profiling(True)
+            c.reset_kernel_times()
+            ref = c.measure(p)
+            assert c.contract_form == 11
+            c.set_profiling(False)
+            for _ in range(2):  # direct, then as a graph
+                b.upload(0, u)
+                b.run()
+                assert np.array_equal(b.result(0), ref)

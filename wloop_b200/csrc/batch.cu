@@ -115,7 +115,8 @@ struct wlg_batch {
     int kernels = 0;  // kernels one run of the phase launches
   } ph[2];
   // per lattice, phase 1: 0 carried lines, 1 temporal gauge with one launch per
-  // extent, 2 with all extents in one walk (FP64: tensor cores; mixed: packed FMAs)
+  // extent, 2 + e with all extents in one walk (FP64: tensor cores, lines scaled by
+  // 2^-e; mixed: packed FMAs, e = 0)
   std::vector<char> use_gram;
   bool use_graph = true;       // capture each phase after its first run and replay it
   int tG = 0, tSB = 0, tBlock = 0, tNCB = 0;  // contraction shape override (tuning)
@@ -389,7 +390,7 @@ template <class T> void build_ops(wlg_batch* b, int phase) {
   }
   cur_phase = 1;
   auto gram_on = [&](int c) { return c < (int)b->use_gram.size() && b->use_gram[c]; };
-  auto walk_on = [&](int c) { return gram_on(c) && b->use_gram[c] == 2; };
+  auto walk_on = [&](int c) { return gram_on(c) && b->use_gram[c] >= 2; };
 
   // ---- loops (wloop.c:524-608) ----
   // temporal-gauge lattices: the first lines, then per R their line step,
@@ -399,6 +400,7 @@ template <class T> void build_ops(wlg_batch* b, int phase) {
     Op op{};
     op.kind = !walk_on(c) ? OP_GRAM_PREP : (b->cfg[c].slices ? OP_SLICES : OP_PAIRS);
     op.cfg = c;
+    op.R = b->use_gram[c] - 2;  // OP_SLICES: the lines' exponent
     sink.push_back(op);
   }
   for (int r = 0; r < maxr; r++)
@@ -610,10 +612,10 @@ template <class T> int issue(wlg_batch* b, int phase) {
         WLG_CUDA(cudaMemsetAsync(acc, 0, f.sp.acc_bytes, ls));
         WLG_CUDA(cudaMemsetAsync(fail, 0, sizeof(unsigned long long), ls));
         for (int ch = 0; ch < f.sp.nchunk; ch++) {
-          slice_lines(f.g, f.sp, ch, uh, bl, hinv, sa, sb, ls);
+          slice_lines(f.g, f.sp, op.R, ch, uh, bl, hinv, sa, sb, ls);
           slice_gram(f.sp, ch, sa, sb, acc, fail, ls);
         }
-        slice_finish(f.g, f.sp, f.bc, acc, (double*)(b->arena + f.wl), ls);
+        slice_finish(f.g, f.sp, op.R, f.bc, acc, (double*)(b->arena + f.wl), ls);
         kernels += 2 + 2 * f.sp.nchunk;
         break;
       }
@@ -677,6 +679,27 @@ template <class T> int issue(wlg_batch* b, int phase) {
     }
   }
   return get_error()[0] ? -1 : kernels;
+}
+
+// The exponent of an FP64 lattice whose lines are not known to stay within the
+// digits' range (slice_exponent), found between the phases from the lines
+// themselves; -1: none, -2: an error.  Phase 1 makes the first lines again.
+int measured_exponent(wlg_batch* b, int c) {
+  const Cfg& f = b->cfg[c];
+  double* uh = (double*)(b->arena + f.gUh);
+  double* bl = (double*)(b->arena + f.gB);
+  const double* hinv = (const double*)(b->arena + f.gH);
+  unsigned long long* top = (unsigned long long*)(b->arena + f.gDev) + 2;
+  gauge_first<double>(f.g, f.gp, f.p.msl,
+                      (const double2*)(b->arena + f.region + 6 * f.D * elem_bytes(b)),
+                      (const double*)(b->arena + f.gG), hinv, uh, bl, nullptr, b->st);
+  slice_largest(f.g, f.sp, uh, bl, hinv, top, b->st);
+  double v = 0.0;
+  if (get_error()[0] ||
+      cudaMemcpyAsync(&v, top, sizeof(v), cudaMemcpyDeviceToHost, b->st) != cudaSuccess ||
+      cudaStreamSynchronize(b->st) != cudaSuccess)
+    return -2;
+  return slice_exponent(v);
 }
 
 // contraction plans and partial-sum offsets (may change with the shape)
@@ -1146,9 +1169,12 @@ int wlg_batch_run(wlg_batch* b) {
     memcpy(dev, b->dev_host + 3 * c, sizeof(dev));
     use[c] = dev[0] <= kGramMaxDeviation;
     const Cfg& f = b->cfg[c];
-    if (use[c] && ((f.slices && slice_in_range(dev[0], dev[1], f.p.mwlr) && slice_prepare(f.sp) == 0) ||
-                   (f.pairs && pair_prepare(f.pairs_scratch ? f.pp_scratch : f.pp) == 0)))
-      use[c] = 2;
+    if (use[c] && f.slices && dev[1] < 300.0 && slice_prepare(f.sp) == 0) {
+      const int e = slice_in_range(dev[0], dev[1], f.p.mwlr) ? 0 : measured_exponent(b, (int)c);
+      if (e == -2) return -1;
+      if (e >= 0) use[c] = (char)(2 + e);
+    }
+    if (use[c] && f.pairs && pair_prepare(f.pairs_scratch ? f.pp_scratch : f.pp) == 0) use[c] = 2;
     set_error("%s", "");
   }
   if (use != b->use_gram) {
@@ -1174,7 +1200,7 @@ int wlg_batch_run(wlg_batch* b) {
     return -1;
   }
   for (size_t c = 0; c < n; c++)
-    if (b->use_gram[c] == 2 && b->dev_host[3 * c + 2] != 0) {
+    if (b->use_gram[c] >= 2 && b->dev_host[3 * c + 2] != 0) {
       set_error("batch_run: the Gram product's operand copies did not arrive in time");
       return -1;
     }

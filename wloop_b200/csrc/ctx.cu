@@ -400,7 +400,7 @@ static void release_idle_scratch(wlg_ctx* c) {
 // the lines of every R as digit planes and their Gram products.  Returns 1
 // (nothing done) when its buffers do not fit.
 static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan& gp,
-                           const SlicePlan& sp, double* wl_mat) {
+                           const SlicePlan& sp, bool in_range, double* wl_mat) {
   const Geo& g = c->g;
   const int msl = p->msl;
   const size_t nb = gp.A * sizeof(double) * 3 * msl;
@@ -418,10 +418,6 @@ static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan&
       return 1;
     }
   }
-  c->used_variant = 11;
-  c->lines_len = 0;
-  c->lines_at = nullptr;
-  c->lines_lazy = p->mwlr >= 2 ? p->mwlr : 0;
   double* uh = (double*)c->gUh.p;
   double* bl = (double*)c->gB.p;
   const double* hinv = (const double*)c->gH.p;
@@ -434,10 +430,25 @@ static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan&
     gauge_first<double>(g, gp, msl, (const double2*)c->levels.p, (const double*)c->gG.p, hinv, uh, bl,
                    nullptr, c->st);
   }
+  int exponent = 0;
+  if (!in_range) {
+    ProfScope ps(c, "gauge");
+    unsigned long long* dtop = (unsigned long long*)c->gDev.p + 1;
+    slice_largest(g, sp, uh, bl, hinv, dtop, c->st);
+    double top = 0.0;
+    WLG_CUDA(cudaMemcpyAsync(&top, dtop, sizeof(top), cudaMemcpyDeviceToHost, c->st));
+    WLG_CUDA(cudaStreamSynchronize(c->st));
+    exponent = slice_exponent(top);
+    if (exponent < 0) return 1;
+  }
+  c->used_variant = 11;
+  c->lines_len = 0;
+  c->lines_at = nullptr;
+  c->lines_lazy = p->mwlr >= 2 ? p->mwlr : 0;
   for (int ch = 0; ch < sp.nchunk; ch++) {
     {
       ProfScope ps(c, "lines");
-      slice_lines(g, sp, ch, uh, bl, hinv, (unsigned char*)c->gSa.p, (unsigned char*)c->gSb.p,
+      slice_lines(g, sp, exponent, ch, uh, bl, hinv, (unsigned char*)c->gSa.p, (unsigned char*)c->gSb.p,
                      c->st);
     }
     {
@@ -447,7 +458,7 @@ static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan&
   }
   {
     ProfScope ps(c, "reduce");
-    slice_finish(g, sp, c->bc, acc, (double*)c->wl.p, c->st);
+    slice_finish(g, sp, exponent, c->bc, acc, (double*)c->wl.p, c->st);
   }
   if (get_error()[0]) return -1;
   int failed = 0;
@@ -571,9 +582,10 @@ static int do_loops_gram(wlg_ctx* c, const wlg_wloop_parms* p, double* wl_mat) {
     WLG_CUDA(cudaStreamSynchronize(c->st));
   }
   if (!(dev[0] <= kGramMaxDeviation)) return 1;
-  slices = slices && slice_in_range(dev[0], dev[1], p->mwlr);
-  if (slices) {
-    const int rc = do_loops_slices(c, p, gp, sp, wl_mat);
+  // (a NaN fails the comparison; links beyond it do not fit any exponent)
+  if (slices && dev[1] < 300.0) {
+    const int rc =
+        do_loops_slices(c, p, gp, sp, slice_in_range(dev[0], dev[1], p->mwlr), wl_mat);
     if (rc != 1) return rc;
   }
   if (pairs) {

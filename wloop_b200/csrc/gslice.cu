@@ -6,11 +6,16 @@
 //     x = sum_p q_p 2^(-6-8p),  q_p in [-128, 127],  p < 7
 //
 // (x rounded to 2^-54; |x| < 1.99).  A line entry is bounded by the product of
-// the operator norms it is made of, so the host admits a lattice only if
+// the operator norms it is made of, so that
 //     (1 + 3 delta)^(R/2) / (1 - 3 dev) <= 1.98
 // (delta, dev: largest |U^dag U - 1| over the stored levels and |g g^dag - 1|
-// over the gauge field); the FMA kernel of gram.cu measures the others, and
-// a NaN anywhere fails the comparison.  A dot product is then
+// over the gauge field) admits a lattice.  Where spatial links are too far from
+// unitary for it (spatial HYP leaves such links), a walk that stores nothing
+// finds the largest entry, and the lines are scaled by 2^-e for the smallest e
+// <= 3 that holds it (32 x 20^3, msl 4, three levels of spatial HYP: 0.35 ms for
+// that walk, against 3.1 ms more in the FMA kernel and its lines: 11.2 to 9.5 ms
+// a measurement); the FMA kernel of gram.cu measures the rest, and a NaN anywhere
+// fails every comparison.  A dot product is then
 //     sum_c a_c b_c = sum_m 2^(-12-8m) C_m,   C_m = sum_{i+j=m} q_a,i . q_b,j
 // over the classes m < 7.  The classes that are left out and the rounding of x
 // are unbiased digits of size 2^-54 per column, and shrink against the sum
@@ -103,17 +108,22 @@ struct Digits {
 // where plane p starts in a lane's 16-byte (o6 for plane 6: o16) column
 __device__ constexpr int plane_at(int p) { return (p >> 1) * 128 + (p & 1) * kKB; }
 
+template <bool SCALED> __device__ __forceinline__ double2 scaled(double2 v, double s) {
+  return SCALED ? make_double2(v.x * s, v.y * s) : v;  // s a power of two
+}
+
 // the digit planes of one matrix into its row (this lane's 16 + 2 bytes per
 // plane); lanes without a site write zeros
+template <bool SCALED>
 __device__ __forceinline__ void store_digits(unsigned char* __restrict__ row, int lane,
-                                             const M3<double>& m, bool live) {
+                                             const M3<double>& m, bool live, double scale) {
   constexpr int P = kPlanes;
   uint4 q[P];
 #pragma unroll
   for (int h = 0; h < 4; h++) {
     unsigned w0[P], w1[P];
-    Digits::half(w0, Digits::raw(m.e[2 * h]));
-    Digits::half(w1, Digits::raw(m.e[2 * h + 1]));
+    Digits::half(w0, Digits::raw(scaled<SCALED>(m.e[2 * h], scale)));
+    Digits::half(w1, Digits::raw(scaled<SCALED>(m.e[2 * h + 1], scale)));
 #pragma unroll
     for (int p = 0; p < P; p++) {
       unsigned v = __byte_perm(w0[p], w1[p], 0x5410);
@@ -126,7 +136,7 @@ __device__ __forceinline__ void store_digits(unsigned char* __restrict__ row, in
     }
   }
   unsigned w[P];
-  Digits::half(w, Digits::raw(m.e[8]));
+  Digits::half(w, Digits::raw(scaled<SCALED>(m.e[8], scale)));
   unsigned char* o16 = row + (lane >> 2) * (6 * kKB) + (lane & 3) * 16;
   unsigned char* s16 = row + kSingle + lane * 16;
   unsigned char* o2 = row + 8 * 6 * kKB + lane * 2;
@@ -159,11 +169,24 @@ struct LineArgs {
   size_t A;  // elements of one slab array
   const double *uh, *bl, *hinv;
   unsigned char *sa, *sb;
+  double scale;             // of the digits (WALK_SCALED)
+  unsigned long long* top;  // largest |entry| as double bits (WALK_MAX)
 };
+enum { WALK_PLAIN, WALK_SCALED, WALK_MAX };
+
+__device__ __forceinline__ void largest(double& top, const M3<double>& m) {
+#pragma unroll
+  for (int e = 0; e < 9; e++) {
+    const double x = fabs(m.e[e].x), y = fabs(m.e[e].y);
+    if (x > top || x != x) top = x;  // a NaN sticks
+    if (y > top || y != y) top = y;
+  }
+}
 
 // B(x, R) and A(x, R) = H^-1(x) B(x, R) H^-1(x + R k) for R = 1..mwlr, as
 // digit planes.  One warp per (y0, unit, level), levels in neighbouring warps
 // (they share the H^-1 tiles), the walk over R in registers.
+template <int WALK>
 __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
   const int lane = threadIdx.x & 31;
   unsigned w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -173,6 +196,7 @@ __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
   const int y0 = (int)(w / a.cur);
   if (y0 >= a.Nu) return;
   const Geo& g = a.g;
+  double top = 0.0;
   const int u = a.u0 + ul, k = u / a.ntile;
   const int jt = unit_tile(g, a.ntile, k, u - k * a.ntile);
   const bool live = jt * 32 + lane < g.vs;
@@ -204,17 +228,29 @@ __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
       y = 0;
       z -= nk * st;
     }
-    store_digits(ob, lane, c, live);
+    if constexpr (WALK == WALK_MAX)
+      largest(top, c);
+    else
+      store_digits<WALK == WALK_SCALED>(ob, lane, c, live, a.scale);
     if (start) {
       ld_slab_as(f, hinv, z >> 5, z & 31);
       mul(t, c, f);
       ld_slab_as(f, hinv, j >> 5, j & 31);
       M3<double> s;
       mul(s, f, t);
-      store_digits(oa, lane, s, live);
+      if constexpr (WALK == WALK_MAX)
+        largest(top, s);
+      else
+        store_digits<WALK == WALK_SCALED>(oa, lane, s, live, a.scale);
     }
     ob += step_b;
     oa += step_a;
+  }
+  if constexpr (WALK == WALK_MAX) {
+    if (top != top) top = 1e300;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if (lane == 0) atomicMax(a.top, (unsigned long long)__double_as_longlong(top));
   }
 }
 
@@ -533,13 +569,13 @@ __global__ void __launch_bounds__(kGramThreads, 1)
 __global__ void __launch_bounds__(256) k_slice_finish(const long long* __restrict__ acc,
                                                       long long nwl, int N0, int mwlt, int mwlr,
                                                       int LL, int open, double norm,
-                                                      double* __restrict__ wl) {
+                                                      double scale, double* __restrict__ wl) {
   for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < nwl;
        o += (long long)gridDim.x * blockDim.x) {
     const int t = (int)((o / LL) % mwlt), x0 = (int)(o / ((long long)LL * mwlt * mwlr));
     double v = 0.0;
     if (!open || x0 + t + 1 < N0) {
-      v = fma((double)acc[o], 0x1p-36, (double)acc[nwl + o] * 0x1p-60) / norm;
+      v = fma((double)acc[o], 0x1p-36 * scale, (double)acc[nwl + o] * (0x1p-60 * scale)) / norm;
     }
     wl[o] = v;
   }
@@ -621,7 +657,8 @@ static void* slice_kernel(int TN) {
 bool slice_plan(SlicePlan& p, const Geo& g, int bc, int msl, int mwlt, int mwlr,
                 size_t budget) {
   p = SlicePlan();
-  if (msl < 1 || msl > 8 || mwlt < 1 || mwlr < 1) return false;
+  // the 64-bit sums hold 70 x 3 N1 N2 N3 products of 2^36
+  if (msl < 1 || msl > 8 || mwlt < 1 || mwlr < 1 || g.vs > 600000) return false;
   p.L = msl;
   p.N0 = g.n[0];
   p.Nu = g.n[0] + (bc == 0 ? 0 : mwlt);
@@ -722,25 +759,54 @@ void levels_deviation(const Geo& g, int msl, const double2* levels,
   WLG_LAUNCH_CHECK("levels_dev");
 }
 
-void slice_lines(const Geo& g, const SlicePlan& p, int chunk, const double* uh,
-                 const double* blines, const double* hinv, unsigned char* sa, unsigned char* sb, cudaStream_t st) {
-  LineArgs a;
+static LineArgs line_args(const Geo& g, const SlicePlan& p, const double* uh, const double* blines,
+                          const double* hinv) {
+  LineArgs a = {};
   a.g = g;
   a.Nu = p.Nu;
   a.ntile = p.ntile;
   a.msl = p.L;
   a.mwlr = p.mwlr;
-  a.u0 = chunk * p.nuc;
-  a.cur = std::min(p.nuc, 3 * p.ntile - a.u0);
   a.nuc = p.nuc;
   a.A = (size_t)p.Nu * p.ntile * kSlabTile;
   a.uh = uh;
   a.bl = blines;
   a.hinv = hinv;
+  return a;
+}
+
+void slice_largest(const Geo& g, const SlicePlan& p, const double* uh, const double* blines,
+                   const double* hinv, unsigned long long* top, cudaStream_t st) {
+  LineArgs a = line_args(g, p, uh, blines, hinv);
+  a.cur = 3 * p.ntile;
+  a.top = top;
+  cudaMemsetAsync(top, 0, sizeof(unsigned long long), st);
+  const long long warps = (long long)p.Nu * a.cur * p.L;
+  k_slice_lines<WALK_MAX><<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(a);
+  WLG_LAUNCH_CHECK("slice_largest");
+}
+
+int slice_exponent(double top) {
+  for (int e = 0; e <= kSliceMaxExponent; e++)
+    if (top <= std::ldexp(1.98, e)) return e;
+  return -1;
+}
+
+void slice_lines(const Geo& g, const SlicePlan& p, int exponent, int chunk, const double* uh,
+                 const double* blines, const double* hinv, unsigned char* sa, unsigned char* sb,
+                 cudaStream_t st) {
+  LineArgs a = line_args(g, p, uh, blines, hinv);
+  a.u0 = chunk * p.nuc;
+  a.cur = std::min(p.nuc, 3 * p.ntile - a.u0);
   a.sa = sa;
   a.sb = sb;
+  a.scale = std::ldexp(1.0, -exponent);
   const long long warps = (long long)p.Nu * a.cur * p.L;
-  k_slice_lines<<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(a);
+  const unsigned grid = (unsigned)((warps + 3) / 4);
+  if (exponent)
+    k_slice_lines<WALK_SCALED><<<grid, 128, 0, st>>>(a);
+  else
+    k_slice_lines<WALK_PLAIN><<<grid, 128, 0, st>>>(a);
   WLG_LAUNCH_CHECK("slice_lines");
 }
 
@@ -780,14 +846,14 @@ void slice_gram(const SlicePlan& p, int chunk, unsigned char* sa, unsigned char*
   WLG_LAUNCH_CHECK("slice_gram");
 }
 
-void slice_finish(const Geo& g, const SlicePlan& p, int bc, const unsigned long long* acc,
-                  double* wl, cudaStream_t st) {
+void slice_finish(const Geo& g, const SlicePlan& p, int exponent, int bc,
+                  const unsigned long long* acc, double* wl, cudaStream_t st) {
   const double norm = 9.0 * g.n[1] * g.n[2] * g.n[3];  // wloop.c:535
   const unsigned grid =
       (unsigned)std::min<size_t>((p.nwl + 255) / 256, (size_t)num_sms() * 16);
   const long long* s = reinterpret_cast<const long long*>(acc);
   k_slice_finish<<<grid, 256, 0, st>>>(s, (long long)p.nwl, p.N0, p.mwlt, p.mwlr, p.L * p.L,
-                                       bc == 0, norm, wl);
+                                       bc == 0, norm, std::ldexp(1.0, 2 * exponent), wl);
   WLG_LAUNCH_CHECK("slice_finish");
 }
 

@@ -206,24 +206,32 @@ struct SlicePlan {
 constexpr size_t kSliceBudget = (size_t)2 << 30;
 bool slice_plan(SlicePlan& p, const Geo& g, int bc, int msl, int mwlt, int mwlr,
                 size_t budget = kSliceBudget);
-// whether every line entry stays within the digits' range, from max |g g^dag - 1|
-// and max |U^dag U - 1| over the levels (false for NaN)
+// whether every line entry is known to stay within the digits' range, from max
+// |g g^dag - 1| and max |U^dag U - 1| over the levels (false for NaN)
 bool slice_in_range(double dev, double delta, int mwlr);
 // shared-memory limit and driver entry point (before any launch or capture)
 int slice_prepare(const SlicePlan& p);
 // *dev (device): max |U^dag U - 1| over the msl levels, as double bits
 void levels_deviation(const Geo& g, int msl, const double2* levels,
                       unsigned long long* dev, cudaStream_t st);
+// *top (device): the largest |entry| of all lines of all extents, as double bits
+void slice_largest(const Geo& g, const SlicePlan& p, const double* uh, const double* blines,
+                   const double* hinv, unsigned long long* top, cudaStream_t st);
+// the smallest e with top <= 1.98 2^e, -1 if it is above the largest allowed (the
+// classes left out grow as 2^(2e) against lines of norm 1)
+constexpr int kSliceMaxExponent = 3;
+int slice_exponent(double top);
 // digit planes of one chunk for R = 1..mwlr from the first lines, the recursion
-// links and H^-1
-void slice_lines(const Geo& g, const SlicePlan& p, int chunk, const double* uh,
-                 const double* blines, const double* hinv, unsigned char* sa, unsigned char* sb, cudaStream_t st);
+// links and H^-1, scaled by 2^-exponent
+void slice_lines(const Geo& g, const SlicePlan& p, int exponent, int chunk, const double* uh,
+                 const double* blines, const double* hinv, unsigned char* sa, unsigned char* sb,
+                 cudaStream_t st);
 // adds the chunk's sums to acc (zeroed before the first chunk); *fail set if a
 // wait ran out
 void slice_gram(const SlicePlan& p, int chunk, unsigned char* sa, unsigned char* sb,
                 unsigned long long* acc, int* fail, cudaStream_t st);
-void slice_finish(const Geo& g, const SlicePlan& p, int bc, const unsigned long long* acc,
-                  double* wl, cudaStream_t st);
+void slice_finish(const Geo& g, const SlicePlan& p, int exponent, int bc,
+                  const unsigned long long* acc, double* wl, cudaStream_t st);
 
 // ---- its mixed-form Gram product in packed FMAs, all extents in one walk
 // (gpair.cu); the runs of columns are those of the GramPlan it is made from ----
