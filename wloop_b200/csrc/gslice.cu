@@ -25,7 +25,7 @@
 // the same fields W is 1.3e-16 .. 4.9e-16 off (2-norm) where the FMA kernel's
 // FP64 sums are 4.1e-16 .. 6.5e-16 off.
 //
-// The mixed form keeps FP32 FMAs in gram.cu: its sums' rounding is part of its
+// The mixed form keeps FP32 FMAs (gpair.cu): its sums' rounding is part of its
 // results.
 //
 // Work is cut into chunks of column units (a unit: one direction, one 32-site
@@ -71,39 +71,31 @@ constexpr int kGramThreads = 192;  // producer warp, MMA warp, four epilogue war
 // digits
 // ---------------------------------------------------------------------------
 // Two roundings by magic addition: t1 = x + 1.5 2^22 rounds x to 2^-30, its low
-// word is round(x 2^30); the remainder (exact, at most 2^-31) plus 0.375 rounds
-// to 2^-54.  The low part may round up to 2^23, its carry goes into the high
-// part.  Bytes below the top one carry a bias of 128, taken off by the flip of
-// their top bit.
+// word is round(x 2^30); the remainder (at most 2^-31) plus 0.375, exact up to
+// the one rounding to 2^-54, holds the rest in its low word.  The low part may
+// round up to 2^23, its carry goes into the high part.  Bytes below the top one
+// carry a bias of 128, taken off by the flip of their top bit.
 struct Digits {
-  struct Raw {
-    unsigned ha, hb, la, lb;
-  };
-  __device__ static __forceinline__ void bits(unsigned& hi, unsigned& lo, double x) {
+  unsigned hi, lo;
+  __device__ explicit __forceinline__ Digits(double x) {
     constexpr double M1 = 6291456.0;  // 1.5 * 2^22: unit in the last place 2^-30
     const double t1 = x + M1;
-    const double m = x - (t1 - M1);
-    const double t2 = m + 0.375;      // unit in the last place 2^-54
+    const double t2 = x - (t1 - (M1 + 0.375));  // unit in the last place 2^-54
     lo = (unsigned)__double2loint(t2) + 0x00808080u;
     hi = (unsigned)__double2loint(t1) + ((int)lo >> 24) + 0x00808080u;
   }
-  __device__ static __forceinline__ Raw raw(double2 v) {
-    Raw x;
-    bits(x.ha, x.la, v.x);
-    bits(x.hb, x.lb, v.y);
-    return x;
-  }
-  __device__ static __forceinline__ void half(unsigned (&w)[kPlanes], const Raw& x) {
-    w[0] = __byte_perm(x.ha, x.hb, 0x0073);
-    w[1] = __byte_perm(x.ha, x.hb, 0x0062);
-    w[2] = __byte_perm(x.ha, x.hb, 0x0051);
-    w[3] = __byte_perm(x.ha, x.hb, 0x0040);
-    w[4] = __byte_perm(x.la, x.lb, 0x0062);
-    w[5] = __byte_perm(x.la, x.lb, 0x0051);
-    w[6] = __byte_perm(x.la, x.lb, 0x0040);
-  }
   static constexpr unsigned flip(int p) { return p == 0 ? 0u : 0x80808080u; }
 };
+
+// the digits of one complex number: planes 0|1, 2|3, 4|5 as the low and high
+// halves of a word (two bytes: real, imaginary), plane 6 as a low half
+__device__ __forceinline__ void digits_of(unsigned (&w)[4], double2 v) {
+  const Digits a(v.x), b(v.y);
+  w[0] = __byte_perm(a.hi, b.hi, 0x6273);
+  w[1] = __byte_perm(a.hi, b.hi, 0x4051);
+  w[2] = __byte_perm(a.lo, b.lo, 0x5162);
+  w[3] = __byte_perm(a.lo, b.lo, 0x0040);
+}
 
 // where plane p starts in a lane's 16-byte (o6 for plane 6: o16) column
 __device__ constexpr int plane_at(int p) { return (p >> 1) * 128 + (p & 1) * kKB; }
@@ -113,30 +105,29 @@ template <bool SCALED> __device__ __forceinline__ double2 scaled(double2 v, doub
 }
 
 // the digit planes of one matrix into its row (this lane's 16 + 2 bytes per
-// plane); lanes without a site write zeros
+// plane)
 template <bool SCALED>
 __device__ __forceinline__ void store_digits(unsigned char* __restrict__ row, int lane,
-                                             const M3<double>& m, bool live, double scale) {
+                                             const M3<double>& m, double scale) {
   constexpr int P = kPlanes;
   uint4 q[P];
 #pragma unroll
   for (int h = 0; h < 4; h++) {
-    unsigned w0[P], w1[P];
-    Digits::half(w0, Digits::raw(scaled<SCALED>(m.e[2 * h], scale)));
-    Digits::half(w1, Digits::raw(scaled<SCALED>(m.e[2 * h + 1], scale)));
+    unsigned w0[4], w1[4];
+    digits_of(w0, scaled<SCALED>(m.e[2 * h], scale));
+    digits_of(w1, scaled<SCALED>(m.e[2 * h + 1], scale));
 #pragma unroll
     for (int p = 0; p < P; p++) {
-      unsigned v = __byte_perm(w0[p], w1[p], 0x5410);
-      if (Digits::flip(p)) v ^= Digits::flip(p);
-      v = live ? v : 0u;
+      const unsigned v =
+          __byte_perm(w0[p >> 1], w1[p >> 1], p & 1 ? 0x7632 : 0x5410) ^ Digits::flip(p);
       if (h == 0) q[p].x = v;
       if (h == 1) q[p].y = v;
       if (h == 2) q[p].z = v;
       if (h == 3) q[p].w = v;
     }
   }
-  unsigned w[P];
-  Digits::half(w, Digits::raw(scaled<SCALED>(m.e[8], scale)));
+  unsigned w[4];
+  digits_of(w, scaled<SCALED>(m.e[8], scale));
   unsigned char* o16 = row + (lane >> 2) * (6 * kKB) + (lane & 3) * 16;
   unsigned char* s16 = row + kSingle + lane * 16;
   unsigned char* o2 = row + 8 * 6 * kKB + lane * 2;
@@ -144,9 +135,9 @@ __device__ __forceinline__ void store_digits(unsigned char* __restrict__ row, in
 #pragma unroll
   for (int p = 0; p < P; p++) {
     *reinterpret_cast<uint4*>(p < 6 ? o16 + plane_at(p) : s16) = q[p];
-    const unsigned v = w[p] ^ (Digits::flip(p) & 0xffffu);
+    const unsigned v = w[p >> 1] ^ (p < 2 ? 0x80800000u : 0x80808080u);
     *reinterpret_cast<unsigned short*>(p < 6 ? o2 + plane_at(p) : s2) =
-        (unsigned short)(live ? v : 0u);
+        (unsigned short)(p & 1 ? v >> 16 : v);
   }
 }
 
@@ -186,6 +177,12 @@ __device__ __forceinline__ void largest(double& top, const M3<double>& m) {
 // B(x, R) and A(x, R) = H^-1(x) B(x, R) H^-1(x + R k) for R = 1..mwlr, as
 // digit planes.  One warp per (y0, unit, level), levels in neighbouring warps
 // (they share the H^-1 tiles), the walk over R in registers.
+//
+// Bound by the writes, 4 KB a matrix: 184 GB and 41-42 ms a measurement at
+// 32^3 x 64 (4.4 TB/s, clocks and bandwidth shared with the Gram product under the
+// power limit).  Neither fewer loads (H^-1(x) B kept in registers), prefetches,
+// streaming stores nor 2 or 4 blocks per SM change it by more than 2 %; three
+// roundings a real instead of four, and no selects, took 3 %.
 template <int WALK>
 __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
   const int lane = threadIdx.x & 31;
@@ -216,6 +213,10 @@ __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
   const size_t step_b = a.nuc * rows_b * kRow, step_a = a.nuc * rows_a * kRow;
   M3<double> c, f, t;
   ld_slab_as(c, a.bl + (size_t)(lev * 3 + k) * a.A + slice, j >> 5, j & 31);
+  if (!live) {  // zero digits in a tile's lanes without a site
+#pragma unroll
+    for (int e = 0; e < 9; e++) c.e[e] = make_double2(0.0, 0.0);
+  }
 #pragma unroll 1
   for (int R = 1; R <= a.mwlr; R++) {
     if (R > 1) {
@@ -231,7 +232,7 @@ __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
     if constexpr (WALK == WALK_MAX)
       largest(top, c);
     else
-      store_digits<WALK == WALK_SCALED>(ob, lane, c, live, a.scale);
+      store_digits<WALK == WALK_SCALED>(ob, lane, c, a.scale);
     if (start) {
       ld_slab_as(f, hinv, z >> 5, z & 31);
       mul(t, c, f);
@@ -241,7 +242,7 @@ __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
       if constexpr (WALK == WALK_MAX)
         largest(top, s);
       else
-        store_digits<WALK == WALK_SCALED>(oa, lane, s, live, a.scale);
+        store_digits<WALK == WALK_SCALED>(oa, lane, s, a.scale);
     }
     ob += step_b;
     oa += step_a;

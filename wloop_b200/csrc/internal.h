@@ -202,8 +202,10 @@ struct SlicePlan {
   size_t bytes_a = 0, bytes_b = 0, acc_bytes = 0, nwl = 0;
 };
 // device memory the digit planes of one chunk may take (false: one column unit
-// needs more)
-constexpr size_t kSliceBudget = (size_t)2 << 30;
+// needs more).  Each chunk costs the ramps and last waves of two kernels, about 40 us
+// each: 32^3 x 64 takes 235 ms at 128 MiB, 211 at 256, 198 at 512, 190 at 1 GiB, 188
+// at 2, 185 at 4, 185 at 8
+constexpr size_t kSliceBudget = (size_t)4 << 30;
 bool slice_plan(SlicePlan& p, const Geo& g, int bc, int msl, int mwlt, int mwlr,
                 size_t budget = kSliceBudget);
 // whether every line entry is known to stay within the digits' range, from max
