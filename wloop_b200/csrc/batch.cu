@@ -140,14 +140,19 @@ namespace {
 // and destroys a batch per group of requests, and cudaMalloc / cudaFree would
 // cost an allocation round trip and a device-wide synchronisation each time,
 // stalling the batches of other workers in flight.
+//
+// A second pool per device holds the scratch that single smearing calls
+// allocate and give back (call_scratch): it keeps at most kCallScratch.
 constexpr int kMaxPoolDevices = 64;
 std::mutex g_pool_mutex;
-cudaMemPool_t g_pool[kMaxPoolDevices] = {nullptr};
+cudaMemPool_t g_pool[2][kMaxPoolDevices] = {};
+enum { kBatchPool, kCallPool };
 
-cudaMemPool_t batch_pool(int dev) {
+cudaMemPool_t device_pool(int which, int dev, bool create) {
   if (dev < 0 || dev >= kMaxPoolDevices) return nullptr;
   std::lock_guard<std::mutex> lock(g_pool_mutex);
-  if (!g_pool[dev]) {
+  cudaMemPool_t& pool = g_pool[which][dev];
+  if (!pool && create) {
     cudaMemPoolProps props;
     memset(&props, 0, sizeof(props));
     props.allocType = cudaMemAllocationTypePinned;
@@ -158,14 +163,30 @@ cudaMemPool_t batch_pool(int dev) {
       cudaGetLastError();
       return nullptr;
     }
-    uint64_t keep = ~0ull;
+    uint64_t keep = which == kBatchPool ? ~0ull : (uint64_t)kCallScratch;
     cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-    g_pool[dev] = p;
+    pool = p;
   }
-  return g_pool[dev];
+  return pool;
 }
 
-// stream-ordered allocation on the batch's stream; on failure the pool's
+void pool_trim(int which, int dev) {
+  if (cudaMemPool_t pool = device_pool(which, dev, false)) cudaMemPoolTrimTo(pool, 0);
+}
+
+long long pool_idle(int which, int dev) {
+  cudaMemPool_t pool = device_pool(which, dev, which == kBatchPool);
+  if (!pool) return 0;
+  uint64_t reserved = 0, used = 0;
+  if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return reserved > used ? (long long)(reserved - used) : 0;
+}
+
+// stream-ordered allocation on the batch's stream; on failure the pools'
 // idle memory is given back to the device and the allocation tried once more
 template <class P>
 int pool_alloc(wlg_batch* b, P** ptr, size_t bytes);
@@ -825,14 +846,14 @@ void layout(wlg_batch* b) {
 template <class P>
 int pool_alloc(wlg_batch* b, P** ptr, size_t bytes) {
   *ptr = nullptr;
-  cudaMemPool_t pool = batch_pool(b->dev);
+  cudaMemPool_t pool = device_pool(kBatchPool, b->dev, true);
   if (!pool) return -1;
   void* p = nullptr;
   cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, b->st);
   if (e != cudaSuccess) {
     cudaGetLastError();
     cudaStreamSynchronize(b->st);
-    cudaMemPoolTrimTo(pool, 0);
+    batch_pool_trim(b->dev);
     e = cudaMallocFromPoolAsync(&p, bytes, pool, b->st);
     if (e != cudaSuccess) {
       cudaGetLastError();
@@ -1059,28 +1080,28 @@ int wlg_batch_destroy(wlg_batch* b) {
 
 namespace wlg {
 void batch_pool_trim(int dev) {
-  if (dev < 0 || dev >= kMaxPoolDevices) return;
-  cudaMemPool_t pool = nullptr;
-  {
-    std::lock_guard<std::mutex> lock(g_pool_mutex);
-    pool = g_pool[dev];
-  }
-  if (pool) cudaMemPoolTrimTo(pool, 0);
+  pool_trim(kBatchPool, dev);
+  pool_trim(kCallPool, dev);
 }
+
+void* call_scratch(int dev, size_t bytes, cudaStream_t st) {
+  void* p = nullptr;
+  cudaMemPool_t pool = device_pool(kCallPool, dev, true);
+  if (!pool) return nullptr;
+  if (cudaMallocFromPoolAsync(&p, bytes, pool, st) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return p;
+}
+
+void call_scratch_trim(int dev) { pool_trim(kCallPool, dev); }
 }  // namespace wlg
 
 extern "C" {
 
 long long wlg_batch_pool_idle_bytes(int device) {
-  cudaMemPool_t pool = batch_pool(device);
-  if (!pool) return 0;
-  uint64_t reserved = 0, used = 0;
-  if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
-      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return reserved > used ? (long long)(reserved - used) : 0;
+  return pool_idle(kBatchPool, device) + pool_idle(kCallPool, device);
 }
 
 int wlg_batch_size(wlg_batch* b) { return b ? (int)b->cfg.size() : 0; }

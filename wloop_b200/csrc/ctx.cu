@@ -53,6 +53,7 @@ using namespace wlg;
 struct DevBuf {
   void* p = nullptr;
   size_t cap = 0;
+  cudaStream_t call = nullptr;  // from call_scratch: the stream to free it on
 };
 
 struct ProfStat {
@@ -96,11 +97,19 @@ struct wlg_ctx {
   int used_variant = 0;  // contraction form of the last measurement
 };
 
-static int ensure(DevBuf& b, size_t bytes) {
-  if (b.cap >= bytes && b.p) return 0;
-  if (b.p) cudaFree(b.p);
+static void release(DevBuf& b) {
+  if (b.call)
+    cudaFreeAsync(b.p, b.call);
+  else if (b.p)
+    cudaFree(b.p);
   b.p = nullptr;
   b.cap = 0;
+  b.call = nullptr;
+}
+
+static int ensure(DevBuf& b, size_t bytes) {
+  if (b.cap >= bytes && b.p) return 0;
+  release(b);
   if (bytes == 0) return 0;
   cudaError_t e = cudaMalloc(&b.p, bytes);
   if (e != cudaSuccess) {
@@ -120,10 +129,19 @@ static int ensure(DevBuf& b, size_t bytes) {
   return 0;
 }
 
-static void release(DevBuf& b) {
-  if (b.p) cudaFree(b.p);
-  b.p = nullptr;
-  b.cap = 0;
+// Scratch that a call without `keep` gives back when it is done: up to
+// kCallScratch a call it comes from the device's pool of such memory (`total`:
+// all that the call takes), unless the context has the buffer from before.
+static int ensure_call(wlg_ctx* c, DevBuf& b, size_t bytes, size_t total, int keep) {
+  if (!keep && !b.p && total <= kCallScratch) {
+    if (void* p = call_scratch(c->dev, bytes, c->st)) {
+      b.p = p;
+      b.cap = bytes;
+      b.call = c->st;
+      return 0;
+    }
+  }
+  return ensure(b, bytes);
 }
 
 // bytes of one direction array (tiled layout, common.cuh) and of ndir of them
@@ -226,7 +244,8 @@ template <class T> static int do_hyp(wlg_ctx* c, double a1, double a2, double a3
                                      int piter, int mu0, int mu1, int keep) {
   if (a1 == 0.0) return 0;  // hyp_links.c:405
   size_t fb = field_bytes(c, 12);
-  if (ensure(c->bar, fb) || ensure(c->til, fb)) return -1;
+  if (ensure_call(c, c->bar, fb, 2 * fb, keep) || ensure_call(c, c->til, fb, 2 * fb, keep))
+    return -1;
   Links<T> U = view4<T>(c->U.p, c->g.vol);
   {
     ProfScope ps(c, "hyp");
@@ -248,7 +267,8 @@ template <class T> static int do_ape(wlg_ctx* c, double alpha, int proj, int pit
                                      int nsweeps, int keep) {
   if (nsweeps <= 0) return 0;
   int mu0 = time ? 0 : 1;
-  if (ensure(c->apeA, field_bytes(c, 4))) return -1;
+  const size_t fb = field_bytes(c, 4);
+  if (ensure_call(c, c->apeA, fb, fb, keep)) return -1;
   Links<T> U = view4<T>(c->U.p, c->g.vol), A = view4<T>(c->apeA.p, c->g.vol);
   {
     ProfScope ps(c, "ape");
@@ -284,6 +304,8 @@ template <class T> static int hyp3_sweep(wlg_ctx* c, Links<T> src, Links<T> dst,
 template <class T> static int do_hyp_spatial(wlg_ctx* c, double a1, double a2, int proj, int piter,
                                              int nsweeps, int keep) {
   Links<T> U = view4<T>(c->U.p, c->g.vol);
+  const size_t fb = field_bytes(c, 6);
+  if (nsweeps > 0 && ensure_call(c, c->dl, fb, fb, keep)) return -1;
   {
     ProfScope ps(c, "hyp3");
     for (int i = 0; i < nsweeps; i++)
@@ -833,6 +855,7 @@ int wlg_free_scratch(wlg_ctx* c) {
   c->lines_lazy = 0;
   release(c->partial);
   release(c->staging);
+  call_scratch_trim(c->dev);
   return 0;
 }
 
@@ -853,6 +876,7 @@ int wlg_destroy(wlg_ctx* c) {
     cudaStreamDestroy(c->cst);
   }
   cudaStreamDestroy(c->st);
+  call_scratch_trim(c->dev);
   delete c;
   return 0;
 }
