@@ -55,7 +55,7 @@ def test_plans(n):
             row = 4096  # 9 x 7 x 64 digits, padded
             assert p["bytes_a"] == r * p["nuc"] * p["rows_a"] * row
             assert p["bytes_b"] == r * p["nuc"] * p["rows_b"] * row
-            assert p["bytes_a"] + p["bytes_b"] <= 2 << 30
+            assert p["bytes_a"] + p["bytes_b"] <= 4 << 30
 
 
 def test_plans_refused():
@@ -65,6 +65,9 @@ def test_plans_refused():
     assert plan(n, 3, 9, 24, 16) is None and plan(n, 3, 6, 0, 16) is None
     assert plan(n, 3, 6, 24, 0) is None and plan(n, 1, 6, 24, 16) is None
     assert plan((8, 1, 4, 4), 3, 2, 2, 2) is None
+    # the 64-bit sums' range
+    assert plan((4, 85, 84, 84), 3, 1, 1, 1) is not None
+    assert plan((4, 86, 84, 84), 3, 1, 1, 1) is None
 
 
 # (lattice, bc, levels, t, r): one A tile with few rows; a row count just past
