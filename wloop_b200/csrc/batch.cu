@@ -13,11 +13,11 @@
 // between the two line buffers; the third form runs a line-step stage.
 // Configurations of at least kGramMinSites sites whose smearing projects
 // (proj_iter >= 3) run the temporal-gauge form (gram.cu) instead, one launch
-// per lattice and stage
-// inside the same graph: its g and H^-1 take the APE ping-pong slots, its A
-// lines the level store (dead once the first lines exist), its recursion
-// links and B lines start at the first line buffer, the region grown where
-// they need more; the carried-line shapes of wlg_batch_set_contract_shape
+// per lattice and stage (gslice.cu, gpair.cu: all extents at once) inside the
+// same graph: its g and H^-1 take the APE ping-pong slots, its digit planes,
+// paired lines or A lines the level store (dead once the first lines exist), its
+// recursion links and B lines start at the first line buffer, the region grown
+// where they need more; the carried-line shapes of wlg_batch_set_contract_shape
 // switch it off.  A run fails if g g^dag of such a lattice is far from 1.
 #include <string.h>
 
