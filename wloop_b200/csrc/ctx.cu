@@ -406,7 +406,9 @@ static int do_smear(wlg_ctx* c, const wlg_wloop_parms* p, double* plaq) {
 // level, host staging) is idle during the loop stage and allocated again by
 // the next measurement that needs it: it is returned to the device when the
 // loop stage's buffers do not fit beside it (FP64 at 48^3x96 holds 58 GB of
-// it).  cudaFree waits for the device, so no copy or kernel still uses it.
+// it).  So are a chunk's lines (4 GiB), which only the form that is about to
+// run would use.  cudaFree waits for the device, so no copy or kernel still
+// uses them.
 static void release_idle_scratch(wlg_ctx* c) {
   release(c->bar);
   release(c->til);
@@ -414,6 +416,8 @@ static void release_idle_scratch(wlg_ctx* c) {
   release(c->apeB);
   release(c->dl);
   release(c->staging);
+  release(c->gSa);
+  release(c->gSb);
   set_error("%s", "");
 }
 
