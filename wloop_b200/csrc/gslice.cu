@@ -607,8 +607,8 @@ __global__ void __launch_bounds__(256) k_levels_dev(const double2* __restrict__ 
         }
         re = fabs(re);
         im = fabs(im);
-        if (!(re <= worst)) worst = re;
-        if (!(im <= worst)) worst = im;
+        if (re > worst || re != re) worst = re;  // a NaN sticks
+        if (im > worst || im != im) worst = im;
       }
   }
   double d = worst != worst ? 1e300 : worst;
