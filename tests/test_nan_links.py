@@ -38,3 +38,19 @@ def test_spatial_link(spot, value):
             b.upload(0, u)
             b.run()
             assert np.array_equal(b.result(0), ref, equal_nan=True)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_temporal_link(precision):
+    """Slices of more than 303104 sites, where also the last slice is shared out in
+    several sites a thread: the gauge field is refused, and the carried lines
+    give NaN from the one start slice whose loops use the link."""
+    n, bc = (2, 68, 68, 68), 3
+    p = WloopParms(msl=2, nss=[0, 0], mwlt=1, mwlr=1, op_smear=APE, alpha_ape=0.5, proj_iter=4)
+    u = generate_links(n, bc, 12, 0.2)
+    u[0, 0] = np.nan
+    with Context(n, bc, precision) as c:
+        c.upload(u)
+        got = c.wloop_sum(p).reshape(n[0], -1)
+        assert c.contract_form != 11
+    assert np.isnan(got[0]).all() and np.isfinite(got[1]).all()

@@ -169,8 +169,8 @@ __global__ void __launch_bounds__(128) k_gauge_inverse(long long nlane, int vs, 
 #pragma unroll
     for (int e = 0; e < 9; e++) {
       const double dr = fabs(t.e[e].x - ((e % 4 == 0) ? 1.0 : 0.0)), di = fabs(t.e[e].y);
-      if (!(dr <= worst)) worst = dr;  // a NaN sticks
-      if (!(di <= worst)) worst = di;
+      if (dr > worst || dr != dr) worst = dr;  // a NaN sticks
+      if (di > worst || di != di) worst = di;
     }
     inverse3(h, t);
     st_slab(Hinv, tile, lane, h);
