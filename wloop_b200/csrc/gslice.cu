@@ -7,9 +7,10 @@
 //
 // (x rounded to 2^-54; |x| < 1.99).  A line entry is bounded by the product of
 // the operator norms it is made of, so that
-//     (1 + 3 delta)^(R/2) / (1 - 3 dev) <= 1.98
-// (delta, dev: largest |U^dag U - 1| over the stored levels and |g g^dag - 1|
-// over the gauge field) admits a lattice.  Where spatial links are too far from
+//     (1 + c delta)^(R/2) / (1 - c dev) <= 1.98,  c = 1 + 2 sqrt 2
+// (delta, dev: largest real or imaginary part of U^dag U - 1 over the stored
+// levels and of g g^dag - 1 over the gauge field; c times it bounds the norm)
+// admits a lattice.  Where spatial links are too far from
 // unitary for it (spatial HYP leaves such links), a walk that stores nothing
 // finds the largest entry, and the lines are scaled by 2^-e for the smallest e
 // <= 3 that holds it (32 x 20^3, msl 4, three levels of spatial HYP: 0.35 ms for
@@ -582,8 +583,8 @@ __global__ void __launch_bounds__(256) k_slice_finish(const long long* __restric
   }
 }
 
-// max |U^dag U - 1| over the stored levels, as the bits of a non-negative
-// double (a NaN counts as the largest value)
+// largest real or imaginary part of U^dag U - 1 over the stored levels, as the bits
+// of a non-negative double (a NaN counts as the largest value)
 __global__ void __launch_bounds__(256) k_levels_dev(const double2* __restrict__ lev,
                                                     size_t stride, int narr, int vol,
                                                     unsigned long long* __restrict__ dev) {
@@ -725,8 +726,12 @@ bool slice_plan(SlicePlan& p, const Geo& g, int bc, int msl, int mwlt, int mwlr,
 }
 
 bool slice_in_range(double dev, double delta, int mwlr) {
-  if (!(dev < 0.3) || !(delta < 0.3)) return false;
-  return std::pow(1.0 + 3.0 * delta, 0.5 * mwlr) / (1.0 - 3.0 * dev) <= 1.98;
+  // a Hermitian matrix whose entries' real and imaginary parts are at most d has a
+  // norm of at most its largest row sum, (1 + 2 sqrt 2) d
+  constexpr double row = 3.8284271247461903;
+  const double s = row * delta, h = row * dev;
+  if (!(s < 1.0) || !(h < 1.0)) return false;
+  return std::pow(1.0 + s, 0.5 * mwlr) / (1.0 - h) <= 1.98;
 }
 
 int slice_prepare(const SlicePlan& p) {
