@@ -3,7 +3,8 @@ others."""
 import numpy as np
 import pytest
 
-from wloop_b200 import APE, Context, WloopParms
+from wloop_b200 import APE, Context, WloopParms, generate_links
+from wloop_b200.api import Batch, launch_count
 
 DELTA = 0.0297  # largest |Re| and |Im| of U^dag U - 1
 
@@ -57,3 +58,26 @@ def test_bound_holds_every_line():
     # lines of R links are at most 1.111^R in norm: sums of 54 x 30^3 products
     columns = 54 * 30 ** 3
     assert np.abs(got - fma).max() <= 4.0 * np.sqrt(columns) * 2.0 ** -53 * 2.25 ** 2
+
+
+@pytest.mark.gpu
+def test_another_scale_replays_the_graph():
+    """A batch's captured graph serves fields whose lines need another scale, and
+    fields that need none: replaying it issues no launches but those that find the
+    scale."""
+    n, bc = (32, 8, 8, 16), 3
+    p = WloopParms(msl=2, nss=[0, 0], mwlt=4, mwlr=2, op_smear=APE, alpha_ape=0.5, proj_iter=4,
+                   alpha_action=(0.0, 1.0, 0.5))
+    base = generate_links(n, bc, 21, 0.05)
+    with Context(n, bc, "fp64") as c, Batch([(n, bc, p)], "fp64") as b:
+        for k, norm in enumerate((1.7, 3.5, 1.2, 1.0, 1.7, 1.0)):
+            u = base.copy()
+            u[:, 1:] *= norm
+            c.upload(u)
+            ref = c.wloop_sum(p)
+            b.upload(0, u)
+            before = launch_count()
+            b.run()
+            if k:
+                assert launch_count() - before <= 2
+            assert np.array_equal(b.result(0), ref)

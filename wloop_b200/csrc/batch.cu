@@ -22,6 +22,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 #include <vector>
 
@@ -115,8 +116,9 @@ struct wlg_batch {
     int kernels = 0;  // kernels one run of the phase launches
   } ph[2];
   // per lattice, phase 1: 0 carried lines, 1 temporal gauge with one launch per
-  // extent, 2 + e with all extents in one walk (FP64: tensor cores, lines scaled by
-  // 2^-e; mixed: packed FMAs, e = 0)
+  // extent, 2 with all extents in one walk (FP64: tensor cores, mixed: packed
+  // FMAs), 3 the same with the FP64 lines scaled by a number in device memory, so
+  // that a field that needs another one runs the same graph
   std::vector<char> use_gram;
   bool use_graph = true;       // capture each phase after its first run and replay it
   int tG = 0, tSB = 0, tBlock = 0, tNCB = 0;  // contraction shape override (tuning)
@@ -421,7 +423,7 @@ template <class T> void build_ops(wlg_batch* b, int phase) {
     Op op{};
     op.kind = !walk_on(c) ? OP_GRAM_PREP : (b->cfg[c].slices ? OP_SLICES : OP_PAIRS);
     op.cfg = c;
-    op.R = b->use_gram[c] - 2;  // OP_SLICES: the lines' exponent
+    op.R = b->use_gram[c];  // OP_SLICES: 3 scales the lines
     sink.push_back(op);
   }
   for (int r = 0; r < maxr; r++)
@@ -632,11 +634,12 @@ template <class T> int issue(wlg_batch* b, int phase) {
         int* fail = (int*)((unsigned long long*)(b->arena + f.gDev) + 2);
         WLG_CUDA(cudaMemsetAsync(acc, 0, f.sp.acc_bytes, ls));
         WLG_CUDA(cudaMemsetAsync(fail, 0, sizeof(unsigned long long), ls));
+        const double* scale = op.R == 3 ? (double*)(b->arena + f.gDev) + 3 : nullptr;
         for (int ch = 0; ch < f.sp.nchunk; ch++) {
-          slice_lines(f.g, f.sp, op.R, ch, uh, bl, hinv, sa, sb, ls);
+          slice_lines(f.g, f.sp, scale, ch, uh, bl, hinv, sa, sb, ls);
           slice_gram(f.sp, ch, sa, sb, acc, fail, ls);
         }
-        slice_finish(f.g, f.sp, op.R, f.bc, acc, (double*)(b->arena + f.wl), ls);
+        slice_finish(f.g, f.sp, scale, f.bc, acc, (double*)(b->arena + f.wl), ls);
         kernels += 2 + 2 * f.sp.nchunk;
         break;
       }
@@ -702,25 +705,33 @@ template <class T> int issue(wlg_batch* b, int phase) {
   return get_error()[0] ? -1 : kernels;
 }
 
-// The exponent of an FP64 lattice whose lines are not known to stay within the
-// digits' range (slice_exponent), found between the phases from the lines
-// themselves; -1: none, -2: an error.  Phase 1 makes the first lines again.
-int measured_exponent(wlg_batch* b, int c) {
+// The scale of an FP64 lattice's lines (slice_exponent), left in device memory: 1
+// where they are known to stay within the digits' range, else found between the
+// phases from the lines themselves.  1: none fits, -1: an error.  Phase 1 makes the
+// first lines again.
+int set_scale(wlg_batch* b, int c, bool in_range) {
   const Cfg& f = b->cfg[c];
-  double* uh = (double*)(b->arena + f.gUh);
-  double* bl = (double*)(b->arena + f.gB);
-  const double* hinv = (const double*)(b->arena + f.gH);
-  unsigned long long* top = (unsigned long long*)(b->arena + f.gDev) + 2;
-  gauge_first<double>(f.g, f.gp, f.p.msl,
-                      (const double2*)(b->arena + f.region + 6 * f.D * elem_bytes(b)),
-                      (const double*)(b->arena + f.gG), hinv, uh, bl, nullptr, b->st);
-  slice_largest(f.g, f.sp, uh, bl, hinv, top, b->st);
-  double v = 0.0;
-  if (get_error()[0] ||
-      cudaMemcpyAsync(&v, top, sizeof(v), cudaMemcpyDeviceToHost, b->st) != cudaSuccess ||
-      cudaStreamSynchronize(b->st) != cudaSuccess)
-    return -2;
-  return slice_exponent(v);
+  double by = 1.0;
+  if (!in_range) {
+    double* uh = (double*)(b->arena + f.gUh);
+    double* bl = (double*)(b->arena + f.gB);
+    const double* hinv = (const double*)(b->arena + f.gH);
+    unsigned long long* top = (unsigned long long*)(b->arena + f.gDev) + 2;
+    gauge_first<double>(f.g, f.gp, f.p.msl,
+                        (const double2*)(b->arena + f.region + 6 * f.D * elem_bytes(b)),
+                        (const double*)(b->arena + f.gG), hinv, uh, bl, nullptr, b->st);
+    slice_largest(f.g, f.sp, uh, bl, hinv, top, b->st);
+    double v = 0.0;
+    if (get_error()[0]) return -1;
+    WLG_CUDA(cudaMemcpyAsync(&v, top, sizeof(v), cudaMemcpyDeviceToHost, b->st));
+    WLG_CUDA(cudaStreamSynchronize(b->st));
+    const int e = slice_exponent(v);
+    if (e < 0) return 1;
+    by = std::ldexp(1.0, -e);
+  }
+  WLG_CUDA(cudaMemcpyAsync((double*)(b->arena + f.gDev) + 3, &by, sizeof(by),
+                           cudaMemcpyHostToDevice, b->st));
+  return 0;
 }
 
 // contraction plans and partial-sum offsets (may change with the shape)
@@ -800,7 +811,7 @@ void layout(wlg_batch* b) {
         o = align256(o + na);
       }
       f.gDev = f.region + o;
-      o = align256(o + 24);
+      o = align256(o + 32);
       // digit planes in the level store; the integer sums
       f.gS = align256(f.region + 6 * f.D * es);
       const size_t room = f.region + lines_at - f.gS;
@@ -1191,9 +1202,12 @@ int wlg_batch_run(wlg_batch* b) {
     use[c] = dev[0] <= kGramMaxDeviation;
     const Cfg& f = b->cfg[c];
     if (use[c] && f.slices && dev[1] < 300.0 && slice_prepare(f.sp) == 0) {
-      const int e = slice_in_range(dev[0], dev[1], f.p.mwlr) ? 0 : measured_exponent(b, (int)c);
-      if (e == -2) return -1;
-      if (e >= 0) use[c] = (char)(2 + e);
+      // a graph that scales the lines serves fields that need no scale too
+      const bool in_range = slice_in_range(dev[0], dev[1], f.p.mwlr);
+      const bool scaled = !in_range || (c < b->use_gram.size() && b->use_gram[c] == 3);
+      const int rc = scaled ? set_scale(b, (int)c, in_range) : 0;
+      if (rc < 0) return -1;
+      if (rc == 0) use[c] = scaled ? 3 : 2;
     }
     if (use[c] && f.pairs && pair_prepare(f.pairs_scratch ? f.pp_scratch : f.pp) == 0) use[c] = 2;
     set_error("%s", "");

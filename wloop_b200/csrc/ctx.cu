@@ -7,6 +7,7 @@
 #include <stdio.h>
 #include <string.h>
 #include <algorithm>
+#include <cmath>
 #include <atomic>
 #include <map>
 #include <string>
@@ -456,7 +457,7 @@ static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan&
     gauge_first<double>(g, gp, msl, (const double2*)c->levels.p, (const double*)c->gG.p, hinv, uh, bl,
                    nullptr, c->st);
   }
-  int exponent = 0;
+  const double* scale = nullptr;
   if (!in_range) {
     ProfScope ps(c, "gauge");
     unsigned long long* dtop = (unsigned long long*)c->gDev.p + 1;
@@ -464,8 +465,12 @@ static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan&
     double top = 0.0;
     WLG_CUDA(cudaMemcpyAsync(&top, dtop, sizeof(top), cudaMemcpyDeviceToHost, c->st));
     WLG_CUDA(cudaStreamSynchronize(c->st));
-    exponent = slice_exponent(top);
+    const int exponent = slice_exponent(top);
     if (exponent < 0) return 1;
+    const double by = std::ldexp(1.0, -exponent);
+    double* at = (double*)c->gDev.p + 3;
+    WLG_CUDA(cudaMemcpyAsync(at, &by, sizeof(by), cudaMemcpyHostToDevice, c->st));
+    scale = at;
   }
   c->used_variant = 11;
   c->lines_len = 0;
@@ -474,8 +479,8 @@ static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan&
   for (int ch = 0; ch < sp.nchunk; ch++) {
     {
       ProfScope ps(c, "lines");
-      slice_lines(g, sp, exponent, ch, uh, bl, hinv, (unsigned char*)c->gSa.p, (unsigned char*)c->gSb.p,
-                     c->st);
+      slice_lines(g, sp, scale, ch, uh, bl, hinv, (unsigned char*)c->gSa.p,
+                  (unsigned char*)c->gSb.p, c->st);
     }
     {
       ProfScope ps(c, "contract");
@@ -484,7 +489,7 @@ static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan&
   }
   {
     ProfScope ps(c, "reduce");
-    slice_finish(g, sp, exponent, c->bc, acc, (double*)c->wl.p, c->st);
+    slice_finish(g, sp, scale, c->bc, acc, (double*)c->wl.p, c->st);
   }
   if (get_error()[0]) return -1;
   int failed = 0;
@@ -595,10 +600,10 @@ static int do_loops_gram(wlg_ctx* c, const wlg_wloop_parms* p, double* wl_mat) {
   const size_t nb = gp.A * sizeof(T) * 3 * msl, na = gp.Aa * sizeof(T) * 3 * msl;
   const size_t nwl = (size_t)msl * msl * p->mwlt * p->mwlr * g.n[0];
   if (ensure(c->gG, gp.A * sizeof(double)) || ensure(c->gH, gp.A * sizeof(double)) ||
-      ensure(c->gDev, 3 * sizeof(unsigned long long)))
+      ensure(c->gDev, 4 * sizeof(unsigned long long)))
     return -1;
   Links<T> U = view4<T>(c->U.p, g.vol);
-  unsigned long long* devs = (unsigned long long*)c->gDev.p;  // dev, delta, failed wait
+  unsigned long long* devs = (unsigned long long*)c->gDev.p;  // dev, delta, failed wait, scale
   double dev[2] = {0.0, 0.0};
   {
     ProfScope ps(c, "gauge");

@@ -161,7 +161,7 @@ struct LineArgs {
   size_t A;  // elements of one slab array
   const double *uh, *bl, *hinv;
   unsigned char *sa, *sb;
-  double scale;             // of the digits (WALK_SCALED)
+  const double* scale;      // of the digits (WALK_SCALED), device memory
   unsigned long long* top;  // largest |entry| as double bits (WALK_MAX)
 };
 enum { WALK_PLAIN, WALK_SCALED, WALK_MAX };
@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
   unsigned char* ob = a.sb + (ul * rows_b + row) * kRow;
   unsigned char* oa = a.sa + (ul * rows_a + row) * kRow;
   const size_t step_b = a.nuc * rows_b * kRow, step_a = a.nuc * rows_a * kRow;
+  const double scale = WALK == WALK_SCALED ? __ldg(a.scale) : 1.0;
   M3<double> c, f, t;
   ld_slab_as(c, a.bl + (size_t)(lev * 3 + k) * a.A + slice, j >> 5, j & 31);
   if (!live) {  // zero digits in a tile's lanes without a site
@@ -233,7 +234,7 @@ __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
     if constexpr (WALK == WALK_MAX)
       largest(top, c);
     else
-      store_digits<WALK == WALK_SCALED>(ob, lane, c, a.scale);
+      store_digits<WALK == WALK_SCALED>(ob, lane, c, scale);
     if (start) {
       ld_slab_as(f, hinv, z >> 5, z & 31);
       mul(t, c, f);
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
       if constexpr (WALK == WALK_MAX)
         largest(top, s);
       else
-        store_digits<WALK == WALK_SCALED>(oa, lane, s, a.scale);
+        store_digits<WALK == WALK_SCALED>(oa, lane, s, scale);
     }
     ob += step_b;
     oa += step_a;
@@ -571,13 +572,15 @@ __global__ void __launch_bounds__(kGramThreads, 1)
 __global__ void __launch_bounds__(256) k_slice_finish(const long long* __restrict__ acc,
                                                       long long nwl, int N0, int mwlt, int mwlr,
                                                       int LL, int open, double norm,
-                                                      double scale, double* __restrict__ wl) {
+                                                      const double* __restrict__ scale,
+                                                      double* __restrict__ wl) {
+  const double lines = scale ? 1.0 / __ldg(scale) : 1.0, both = lines * lines;
   for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < nwl;
        o += (long long)gridDim.x * blockDim.x) {
     const int t = (int)((o / LL) % mwlt), x0 = (int)(o / ((long long)LL * mwlt * mwlr));
     double v = 0.0;
     if (!open || x0 + t + 1 < N0) {
-      v = fma((double)acc[o], 0x1p-36 * scale, (double)acc[nwl + o] * (0x1p-60 * scale)) / norm;
+      v = fma((double)acc[o], 0x1p-36 * both, (double)acc[nwl + o] * (0x1p-60 * both)) / norm;
     }
     wl[o] = v;
   }
@@ -798,18 +801,18 @@ int slice_exponent(double top) {
   return -1;
 }
 
-void slice_lines(const Geo& g, const SlicePlan& p, int exponent, int chunk, const double* uh,
-                 const double* blines, const double* hinv, unsigned char* sa, unsigned char* sb,
-                 cudaStream_t st) {
+void slice_lines(const Geo& g, const SlicePlan& p, const double* scale, int chunk,
+                 const double* uh, const double* blines, const double* hinv, unsigned char* sa,
+                 unsigned char* sb, cudaStream_t st) {
   LineArgs a = line_args(g, p, uh, blines, hinv);
   a.u0 = chunk * p.nuc;
   a.cur = std::min(p.nuc, 3 * p.ntile - a.u0);
   a.sa = sa;
   a.sb = sb;
-  a.scale = std::ldexp(1.0, -exponent);
+  a.scale = scale;
   const long long warps = (long long)p.Nu * a.cur * p.L;
   const unsigned grid = (unsigned)((warps + 3) / 4);
-  if (exponent)
+  if (scale)
     k_slice_lines<WALK_SCALED><<<grid, 128, 0, st>>>(a);
   else
     k_slice_lines<WALK_PLAIN><<<grid, 128, 0, st>>>(a);
@@ -852,14 +855,14 @@ void slice_gram(const SlicePlan& p, int chunk, unsigned char* sa, unsigned char*
   WLG_LAUNCH_CHECK("slice_gram");
 }
 
-void slice_finish(const Geo& g, const SlicePlan& p, int exponent, int bc,
+void slice_finish(const Geo& g, const SlicePlan& p, const double* scale, int bc,
                   const unsigned long long* acc, double* wl, cudaStream_t st) {
   const double norm = 9.0 * g.n[1] * g.n[2] * g.n[3];  // wloop.c:535
   const unsigned grid =
       (unsigned)std::min<size_t>((p.nwl + 255) / 256, (size_t)num_sms() * 16);
   const long long* s = reinterpret_cast<const long long*>(acc);
   k_slice_finish<<<grid, 256, 0, st>>>(s, (long long)p.nwl, p.N0, p.mwlt, p.mwlr, p.L * p.L,
-                                       bc == 0, norm, std::ldexp(1.0, 2 * exponent), wl);
+                                       bc == 0, norm, scale, wl);
   WLG_LAUNCH_CHECK("slice_finish");
 }
 

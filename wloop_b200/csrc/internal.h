@@ -224,15 +224,15 @@ void slice_largest(const Geo& g, const SlicePlan& p, const double* uh, const dou
 constexpr int kSliceMaxExponent = 3;
 int slice_exponent(double top);
 // digit planes of one chunk for R = 1..mwlr from the first lines, the recursion
-// links and H^-1, scaled by 2^-exponent
-void slice_lines(const Geo& g, const SlicePlan& p, int exponent, int chunk, const double* uh,
-                 const double* blines, const double* hinv, unsigned char* sa, unsigned char* sb,
-                 cudaStream_t st);
+// links and H^-1, times *scale (device; a power of two, null: 1)
+void slice_lines(const Geo& g, const SlicePlan& p, const double* scale, int chunk,
+                 const double* uh, const double* blines, const double* hinv, unsigned char* sa,
+                 unsigned char* sb, cudaStream_t st);
 // adds the chunk's sums to acc (zeroed before the first chunk); *fail set if a
 // wait ran out
 void slice_gram(const SlicePlan& p, int chunk, unsigned char* sa, unsigned char* sb,
                 unsigned long long* acc, int* fail, cudaStream_t st);
-void slice_finish(const Geo& g, const SlicePlan& p, int exponent, int bc,
+void slice_finish(const Geo& g, const SlicePlan& p, const double* scale, int bc,
                   const unsigned long long* acc, double* wl, cudaStream_t st);
 
 // ---- its mixed-form Gram product in packed FMAs, all extents in one walk
