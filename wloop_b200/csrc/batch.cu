@@ -52,7 +52,7 @@ struct Cfg {
   // store, dead once the first lines exist
   bool slices;
   SlicePlan sp;
-  size_t gS, gAcc;
+  size_t gS, gAcc, gRange;
   // the mixed form's packed Gram product (gpair.cu): its lines and partial sums
   // take the level store too, or the scratch of the lattice's stream where the
   // store is small and the scratch could be had
@@ -117,8 +117,8 @@ struct wlg_batch {
   } ph[2];
   // per lattice, phase 1: 0 carried lines, 1 temporal gauge with one launch per
   // extent, 2 with all extents in one walk (FP64: tensor cores, mixed: packed
-  // FMAs), 3 the same with the FP64 lines scaled by a number in device memory, so
-  // that a field that needs another one runs the same graph
+  // FMAs), 3 the same with the FP64 lines scaled by numbers in device memory, so
+  // that a field that needs others runs the same graph
   std::vector<char> use_gram;
   bool use_graph = true;       // capture each phase after its first run and replay it
   int tG = 0, tSB = 0, tBlock = 0, tNCB = 0;  // contraction shape override (tuning)
@@ -554,6 +554,10 @@ template <class T> void build_ops(wlg_batch* b, int phase) {
   b->ph[phase].host_tables.swap(tb.bytes);
 }
 
+double* scales_of(wlg_batch* b, const Cfg& f) {
+  return (double*)(b->arena + f.gRange + slice_range_bytes(f.sp));
+}
+
 template <class T> int issue(wlg_batch* b, int phase) {
   int kernels = 0;
   const char* tables = b->ph[phase].tables;
@@ -634,7 +638,7 @@ template <class T> int issue(wlg_batch* b, int phase) {
         int* fail = (int*)((unsigned long long*)(b->arena + f.gDev) + 2);
         WLG_CUDA(cudaMemsetAsync(acc, 0, f.sp.acc_bytes, ls));
         WLG_CUDA(cudaMemsetAsync(fail, 0, sizeof(unsigned long long), ls));
-        const double* scale = op.R == 3 ? (double*)(b->arena + f.gDev) + 3 : nullptr;
+        const double* scale = op.R == 3 ? scales_of(b, f) : nullptr;
         for (int ch = 0; ch < f.sp.nchunk; ch++) {
           slice_lines(f.g, f.sp, scale, ch, uh, bl, hinv, sa, sb, ls);
           slice_gram(f.sp, ch, sa, sb, acc, fail, ls);
@@ -705,32 +709,32 @@ template <class T> int issue(wlg_batch* b, int phase) {
   return get_error()[0] ? -1 : kernels;
 }
 
-// The scale of an FP64 lattice's lines (slice_exponent), left in device memory: 1
-// where they are known to stay within the digits' range, else found between the
-// phases from the lines themselves.  1: none fits, -1: an error.  Phase 1 makes the
-// first lines again.
-int set_scale(wlg_batch* b, int c, bool in_range) {
+// The scales of an FP64 lattice's lines (slice_scales), left in device memory: 1
+// where the lines are known to stay within the digits' range, else found between
+// the phases from the lines themselves.  1: none fit, -1: an error.  Phase 1 makes
+// the first lines again.
+int set_scales(wlg_batch* b, int c, bool in_range) {
   const Cfg& f = b->cfg[c];
-  double by = 1.0;
+  std::vector<double> by((size_t)f.p.mwlr * f.p.msl, 1.0);
   if (!in_range) {
     double* uh = (double*)(b->arena + f.gUh);
     double* bl = (double*)(b->arena + f.gB);
     const double* hinv = (const double*)(b->arena + f.gH);
-    unsigned long long* top = (unsigned long long*)(b->arena + f.gDev) + 2;
+    unsigned long long* range = (unsigned long long*)(b->arena + f.gRange);
     gauge_first<double>(f.g, f.gp, f.p.msl,
                         (const double2*)(b->arena + f.region + 6 * f.D * elem_bytes(b)),
                         (const double*)(b->arena + f.gG), hinv, uh, bl, nullptr, b->st);
-    slice_largest(f.g, f.sp, uh, bl, hinv, top, b->st);
-    double v = 0.0;
+    slice_ranges(f.g, f.sp, uh, bl, hinv, range, b->st);
     if (get_error()[0]) return -1;
-    WLG_CUDA(cudaMemcpyAsync(&v, top, sizeof(v), cudaMemcpyDeviceToHost, b->st));
+    std::vector<unsigned long long> seen(slice_range_bytes(f.sp) / sizeof(unsigned long long));
+    WLG_CUDA(cudaMemcpyAsync(seen.data(), range, slice_range_bytes(f.sp), cudaMemcpyDeviceToHost,
+                             b->st));
     WLG_CUDA(cudaStreamSynchronize(b->st));
-    const int e = slice_exponent(v);
-    if (e < 0) return 1;
-    by = std::ldexp(1.0, -e);
+    if (!slice_scales(f.g, f.sp, f.gp.cpc * 32, f.gp.nsplit, seen.data(), by.data())) return 1;
   }
-  WLG_CUDA(cudaMemcpyAsync((double*)(b->arena + f.gDev) + 3, &by, sizeof(by),
+  WLG_CUDA(cudaMemcpyAsync(scales_of(b, f), by.data(), by.size() * sizeof(double),
                            cudaMemcpyHostToDevice, b->st));
+  WLG_CUDA(cudaStreamSynchronize(b->st));
   return 0;
 }
 
@@ -811,7 +815,7 @@ void layout(wlg_batch* b) {
         o = align256(o + na);
       }
       f.gDev = f.region + o;
-      o = align256(o + 32);
+      o = align256(o + 24);
       // digit planes in the level store; the integer sums
       f.gS = align256(f.region + 6 * f.D * es);
       const size_t room = f.region + lines_at - f.gS;
@@ -819,6 +823,8 @@ void layout(wlg_batch* b) {
                                            std::min(room - 512, kSliceBudget))) {
         f.gAcc = f.region + o;
         o = align256(o + f.sp.acc_bytes);
+        f.gRange = f.region + o;  // then the scales
+        o = align256(o + slice_range_bytes(f.sp) + sizeof(double) * f.p.mwlr * f.p.msl);
       } else {
         f.sp = SlicePlan();
       }
@@ -1203,9 +1209,9 @@ int wlg_batch_run(wlg_batch* b) {
     const Cfg& f = b->cfg[c];
     if (use[c] && f.slices && dev[1] < 300.0 && slice_prepare(f.sp) == 0) {
       // a graph that scales the lines serves fields that need no scale too
-      const bool in_range = slice_in_range(dev[0], dev[1], f.p.mwlr);
+      const bool in_range = slice_in_range(dev[0], dev[1], f.p.mwlr, f.gp.cpc * 32, f.gp.nsplit);
       const bool scaled = !in_range || (c < b->use_gram.size() && b->use_gram[c] == 3);
-      const int rc = scaled ? set_scale(b, (int)c, in_range) : 0;
+      const int rc = scaled ? set_scales(b, (int)c, in_range) : 0;
       if (rc < 0) return -1;
       if (rc == 0) use[c] = scaled ? 3 : 2;
     }

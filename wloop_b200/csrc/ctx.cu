@@ -72,8 +72,8 @@ struct wlg_ctx {
   // unitarity deviation of g
   DevBuf gG, gH, gUh, gB, gA, gDev;
   // the lines of one chunk of columns, all extents (digit planes or FP32 level
-  // pairs), and the tensor-core product's integer sums
-  DevBuf gSa, gSb, gAcc;
+  // pairs), the tensor-core product's integer sums, and its lines' range and scales
+  DevBuf gSa, gSb, gAcc, gRange;
   void* lines_at = nullptr;  // buffer holding the lines of length lines_len
   // after a temporal-gauge measurement the lines of length lines_lazy are
   // rebuilt from the level store when they are asked for
@@ -431,9 +431,11 @@ static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan&
   const Geo& g = c->g;
   const int msl = p->msl;
   const size_t nb = gp.A * sizeof(double) * 3 * msl;
+  const size_t range_bytes = slice_range_bytes(sp);
   auto alloc = [&]() {
     return ensure(c->gUh, nb) || ensure(c->gB, nb) || ensure(c->gSa, sp.bytes_a) ||
            ensure(c->gSb, sp.bytes_b) || ensure(c->gAcc, sp.acc_bytes) ||
+           (!in_range && ensure(c->gRange, range_bytes + sizeof(double) * p->mwlr * msl)) ||
            ensure(c->wl, sizeof(double) * sp.nwl);
   };
   if (alloc()) {
@@ -460,16 +462,17 @@ static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan&
   const double* scale = nullptr;
   if (!in_range) {
     ProfScope ps(c, "gauge");
-    unsigned long long* dtop = (unsigned long long*)c->gDev.p + 1;
-    slice_largest(g, sp, uh, bl, hinv, dtop, c->st);
-    double top = 0.0;
-    WLG_CUDA(cudaMemcpyAsync(&top, dtop, sizeof(top), cudaMemcpyDeviceToHost, c->st));
+    unsigned long long* range = (unsigned long long*)c->gRange.p;
+    slice_ranges(g, sp, uh, bl, hinv, range, c->st);
+    std::vector<unsigned long long> seen(range_bytes / sizeof(unsigned long long));
+    std::vector<double> scales((size_t)p->mwlr * msl);
+    WLG_CUDA(cudaMemcpyAsync(seen.data(), range, range_bytes, cudaMemcpyDeviceToHost, c->st));
     WLG_CUDA(cudaStreamSynchronize(c->st));
-    const int exponent = slice_exponent(top);
-    if (exponent < 0) return 1;
-    const double by = std::ldexp(1.0, -exponent);
-    double* at = (double*)c->gDev.p + 3;
-    WLG_CUDA(cudaMemcpyAsync(at, &by, sizeof(by), cudaMemcpyHostToDevice, c->st));
+    if (!slice_scales(g, sp, gp.cpc * 32, gp.nsplit, seen.data(), scales.data())) return 1;
+    double* at = (double*)((char*)range + range_bytes);
+    WLG_CUDA(cudaMemcpyAsync(at, scales.data(), scales.size() * sizeof(double),
+                             cudaMemcpyHostToDevice, c->st));
+    WLG_CUDA(cudaStreamSynchronize(c->st));
     scale = at;
   }
   c->used_variant = 11;
@@ -600,10 +603,10 @@ static int do_loops_gram(wlg_ctx* c, const wlg_wloop_parms* p, double* wl_mat) {
   const size_t nb = gp.A * sizeof(T) * 3 * msl, na = gp.Aa * sizeof(T) * 3 * msl;
   const size_t nwl = (size_t)msl * msl * p->mwlt * p->mwlr * g.n[0];
   if (ensure(c->gG, gp.A * sizeof(double)) || ensure(c->gH, gp.A * sizeof(double)) ||
-      ensure(c->gDev, 4 * sizeof(unsigned long long)))
+      ensure(c->gDev, 3 * sizeof(unsigned long long)))
     return -1;
   Links<T> U = view4<T>(c->U.p, g.vol);
-  unsigned long long* devs = (unsigned long long*)c->gDev.p;  // dev, delta, failed wait, scale
+  unsigned long long* devs = (unsigned long long*)c->gDev.p;  // dev, delta, failed wait
   double dev[2] = {0.0, 0.0};
   {
     ProfScope ps(c, "gauge");
@@ -615,8 +618,8 @@ static int do_loops_gram(wlg_ctx* c, const wlg_wloop_parms* p, double* wl_mat) {
   if (!(dev[0] <= kGramMaxDeviation)) return 1;
   // (a NaN fails the comparison; links beyond it do not fit any exponent)
   if (slices && dev[1] < 300.0) {
-    const int rc =
-        do_loops_slices(c, p, gp, sp, slice_in_range(dev[0], dev[1], p->mwlr), wl_mat);
+    const bool in_range = slice_in_range(dev[0], dev[1], p->mwlr, gp.cpc * 32, gp.nsplit);
+    const int rc = do_loops_slices(c, p, gp, sp, in_range, wl_mat);
     if (rc != 1) return rc;
   }
   if (pairs) {
@@ -859,6 +862,7 @@ int wlg_free_scratch(wlg_ctx* c) {
   release(c->gSa);
   release(c->gSb);
   release(c->gAcc);
+  release(c->gRange);
   c->lines_at = nullptr;
   c->lines_len = 0;
   c->lines_lazy = 0;
@@ -875,7 +879,7 @@ int wlg_destroy(wlg_ctx* c) {
   if (c->cst) cudaStreamSynchronize(c->cst);
   harvest(c);
   DevBuf* all[] = {&c->U, &c->U0, &c->bar, &c->til, &c->apeA, &c->apeB, &c->dl, &c->levels, &c->lines, &c->lines2,
-                   &c->gG, &c->gH, &c->gUh, &c->gB, &c->gA, &c->gDev, &c->gSa, &c->gSb, &c->gAcc, &c->partial, &c->wl, &c->plaq_part, &c->plaq_out, &c->plaq_count, &c->staging, &c->ipt,
+                   &c->gG, &c->gH, &c->gUh, &c->gB, &c->gA, &c->gDev, &c->gSa, &c->gSb, &c->gAcc, &c->gRange, &c->partial, &c->wl, &c->plaq_part, &c->plaq_out, &c->plaq_count, &c->staging, &c->ipt,
                    &c->prefetch_buf};
   for (DevBuf* b : all) release(*b);
   for (cudaEvent_t e : c->evpool) cudaEventDestroy(e);

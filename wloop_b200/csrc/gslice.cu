@@ -12,11 +12,11 @@
 // levels and of g g^dag - 1 over the gauge field; c times it bounds the norm)
 // admits a lattice.  Where spatial links are too far from
 // unitary for it (spatial HYP leaves such links), a walk that stores nothing
-// finds the largest entry, and the lines are scaled by 2^-e for the smallest e
-// <= 3 that holds it (32 x 20^3, msl 4, three levels of spatial HYP: 0.35 ms for
-// that walk, against 3.1 ms more in the FMA kernel and its lines: 11.2 to 9.5 ms
-// a measurement); the FMA kernel of gram.cu measures the rest, and a NaN anywhere
-// fails every comparison.  A dot product is then
+// finds the largest entry and the least norm of a slice per extent and level, and
+// the lines of each extent and level are scaled by 2^-e for the smallest e <= 3
+// that holds them, unless their norm is so far below it that FP64 FMAs would be
+// nearer (slice_scales).  The FMA kernel of gram.cu measures the rest, and a NaN
+// anywhere fails every comparison.  A dot product is then
 //     sum_c a_c b_c = sum_m 2^(-12-8m) C_m,   C_m = sum_{i+j=m} q_a,i . q_b,j
 // over the classes m < 7.  The classes that are left out and the rounding of x
 // are unbiased digits of size 2^-54 per column, and shrink against the sum
@@ -49,6 +49,7 @@
 // knows, a warp one contiguous row.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <mutex>
 #include <set>
 #include <utility>
@@ -161,17 +162,32 @@ struct LineArgs {
   size_t A;  // elements of one slab array
   const double *uh, *bl, *hinv;
   unsigned char *sa, *sb;
-  const double* scale;      // of the digits (WALK_SCALED), device memory
-  unsigned long long* top;  // largest |entry| as double bits (WALK_MAX)
+  const double* scale;        // [extent][level] (WALK_SCALED)
+  unsigned long long* range;  // see slice_range_bytes (WALK_RANGE)
 };
-enum { WALK_PLAIN, WALK_SCALED, WALK_MAX };
+enum { WALK_PLAIN, WALK_SCALED, WALK_RANGE };
 
-__device__ __forceinline__ void largest(double& top, const M3<double>& m) {
+// this warp's share of one extent's range: the largest entry (its high word, for
+// NaN and infinity above every finite one) and the sum of squares in units of
+// 2^-30, as integers so that their order does not matter
+__device__ __forceinline__ void add_range(unsigned long long* top, unsigned long long* sum,
+                                          const M3<double>& m, bool live, int lane) {
+  unsigned hi = 0;
+  double sq = 0.0;
 #pragma unroll
   for (int e = 0; e < 9; e++) {
-    const double x = fabs(m.e[e].x), y = fabs(m.e[e].y);
-    if (x > top || x != x) top = x;  // a NaN sticks
-    if (y > top || y != y) top = y;
+    hi = max(hi, max((unsigned)__double2hiint(m.e[e].x) & 0x7fffffffu,
+                     (unsigned)__double2hiint(m.e[e].y) & 0x7fffffffu));
+    sq = fma(m.e[e].x, m.e[e].x, fma(m.e[e].y, m.e[e].y, sq));
+  }
+  hi = __reduce_max_sync(0xffffffffu, live ? hi : 0u);
+  if (!live) sq = 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+  if (lane == 0) {
+    if (hi > *(volatile unsigned long long*)top) atomicMax(top, (unsigned long long)hi);
+    // (at most 2^18 where every entry fits the largest exponent)
+    atomicAdd(sum, (unsigned long long)(fmin(sq, 0x1p18) * 0x1p30));
   }
 }
 
@@ -194,7 +210,6 @@ __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
   const int y0 = (int)(w / a.cur);
   if (y0 >= a.Nu) return;
   const Geo& g = a.g;
-  double top = 0.0;
   const int u = a.u0 + ul, k = u / a.ntile;
   const int jt = unit_tile(g, a.ntile, k, u - k * a.ntile);
   const bool live = jt * 32 + lane < g.vs;
@@ -212,7 +227,6 @@ __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
   unsigned char* ob = a.sb + (ul * rows_b + row) * kRow;
   unsigned char* oa = a.sa + (ul * rows_a + row) * kRow;
   const size_t step_b = a.nuc * rows_b * kRow, step_a = a.nuc * rows_a * kRow;
-  const double scale = WALK == WALK_SCALED ? __ldg(a.scale) : 1.0;
   M3<double> c, f, t;
   ld_slab_as(c, a.bl + (size_t)(lev * 3 + k) * a.A + slice, j >> 5, j & 31);
   if (!live) {  // zero digits in a tile's lanes without a site
@@ -231,8 +245,11 @@ __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
       y = 0;
       z -= nk * st;
     }
-    if constexpr (WALK == WALK_MAX)
-      largest(top, c);
+    const int el = (R - 1) * a.msl + lev;
+    const double scale = WALK == WALK_SCALED ? __ldg(a.scale + el) : 1.0;
+    unsigned long long* sums = a.range + (size_t)a.mwlr * a.msl + (size_t)el * 2 * a.Nu + y0;
+    if constexpr (WALK == WALK_RANGE)
+      add_range(a.range + el, sums, c, live, lane);
     else
       store_digits<WALK == WALK_SCALED>(ob, lane, c, scale);
     if (start) {
@@ -241,19 +258,13 @@ __global__ void __launch_bounds__(128, 3) k_slice_lines(LineArgs a) {
       ld_slab_as(f, hinv, j >> 5, j & 31);
       M3<double> s;
       mul(s, f, t);
-      if constexpr (WALK == WALK_MAX)
-        largest(top, s);
+      if constexpr (WALK == WALK_RANGE)
+        add_range(a.range + el, sums + a.Nu, s, live, lane);
       else
         store_digits<WALK == WALK_SCALED>(oa, lane, s, scale);
     }
     ob += step_b;
     oa += step_a;
-  }
-  if constexpr (WALK == WALK_MAX) {
-    if (top != top) top = 1e300;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
-    if (lane == 0) atomicMax(a.top, (unsigned long long)__double_as_longlong(top));
   }
 }
 
@@ -571,15 +582,18 @@ __global__ void __launch_bounds__(kGramThreads, 1)
 // exact zeros
 __global__ void __launch_bounds__(256) k_slice_finish(const long long* __restrict__ acc,
                                                       long long nwl, int N0, int mwlt, int mwlr,
-                                                      int LL, int open, double norm,
+                                                      int L, int open, double norm,
                                                       const double* __restrict__ scale,
                                                       double* __restrict__ wl) {
-  const double lines = scale ? 1.0 / __ldg(scale) : 1.0, both = lines * lines;
   for (long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x; o < nwl;
        o += (long long)gridDim.x * blockDim.x) {
-    const int t = (int)((o / LL) % mwlt), x0 = (int)(o / ((long long)LL * mwlt * mwlr));
+    const int s1 = (int)(o % L), s2 = (int)((o / L) % L), t = (int)((o / (L * L)) % mwlt);
+    const int r = (int)((o / ((long long)L * L * mwlt)) % mwlr);
+    const int x0 = (int)(o / ((long long)L * L * mwlt * mwlr));
     double v = 0.0;
     if (!open || x0 + t + 1 < N0) {
+      const double both =
+          scale ? 1.0 / (__ldg(scale + r * L + s1) * __ldg(scale + r * L + s2)) : 1.0;
       v = fma((double)acc[o], 0x1p-36 * both, (double)acc[nwl + o] * (0x1p-60 * both)) / norm;
     }
     wl[o] = v;
@@ -728,13 +742,51 @@ bool slice_plan(SlicePlan& p, const Geo& g, int bc, int msl, int mwlt, int mwlr,
   return true;
 }
 
-bool slice_in_range(double dev, double delta, int mwlr) {
+// Lines whose digits' unit is 2^-54 c (c: 2^e over the lines' norm) make sums 9 c^2 /
+// sqrt(run + runs) times as far off as FP64 FMAs of `run` columns each, `runs` of
+// them added up: 0.04 to 0.33 at c = 1 for the plans of 32768 sites and more. The
+// largest c^2 that keeps the digits ahead, and 1.1 for the lines of SU(3) links.
+static double most_spread(int run, int runs) {
+  return std::max(1.1, 0.08 * std::sqrt((double)run + runs));
+}
+
+bool slice_in_range(double dev, double delta, int mwlr, int run, int runs) {
   // a Hermitian matrix whose entries' real and imaginary parts are at most d has a
   // norm of at most its largest row sum, (1 + 2 sqrt 2) d
   constexpr double row = 3.8284271247461903;
   const double s = row * delta, h = row * dev;
   if (!(s < 1.0) || !(h < 1.0)) return false;
-  return std::pow(1.0 + s, 0.5 * mwlr) / (1.0 - h) <= 1.98;
+  const double least = std::pow(1.0 - s, 0.5 * mwlr) * (1.0 - h);  // norm of a line
+  return std::pow(1.0 + s, 0.5 * mwlr) / (1.0 - h) <= 1.98 &&
+         1.0 <= most_spread(run, runs) * least * least;
+}
+
+size_t slice_range_bytes(const SlicePlan& p) {
+  return (size_t)p.mwlr * p.L * (1 + 2 * (size_t)p.Nu) * sizeof(unsigned long long);
+}
+
+bool slice_scales(const Geo& g, const SlicePlan& p, int run, int runs,
+                  const unsigned long long* range, double* scale) {
+  const double most = most_spread(run, runs);
+  const unsigned long long* sums = range + (size_t)p.mwlr * p.L;
+  for (int el = 0; el < p.mwlr * p.L; el++) {
+    // above every entry with this high word
+    const unsigned long long bits = (range[el] + 1) << 32;
+    double top;
+    memcpy(&top, &bits, sizeof(top));
+    int e;
+    if (range[el] >= 0x7ff00000ull || !(top <= std::ldexp(1.98, kSliceMaxExponent))) return false;
+    std::frexp(top / 1.98, &e);  // top <= 1.98 2^e
+    scale[el] = std::ldexp(1.0, -e);
+    // the slice of least norm, against lines in SU(3) (three units a matrix)
+    unsigned long long least = ~0ull;
+    for (int y0 = 0; y0 < p.Nu; y0++) least = std::min(least, sums[(size_t)el * 2 * p.Nu + y0]);
+    for (int y0 = 0; y0 < p.N0; y0++)
+      least = std::min(least, sums[(size_t)(el * 2 + 1) * p.Nu + y0]);
+    const double norm2 = std::ldexp((double)least, -30) / (9.0 * g.vs);
+    if (!(std::ldexp(1.0, 2 * e) <= most * norm2)) return false;
+  }
+  return true;
 }
 
 int slice_prepare(const SlicePlan& p) {
@@ -784,21 +836,15 @@ static LineArgs line_args(const Geo& g, const SlicePlan& p, const double* uh, co
   return a;
 }
 
-void slice_largest(const Geo& g, const SlicePlan& p, const double* uh, const double* blines,
-                   const double* hinv, unsigned long long* top, cudaStream_t st) {
+void slice_ranges(const Geo& g, const SlicePlan& p, const double* uh, const double* blines,
+                  const double* hinv, unsigned long long* range, cudaStream_t st) {
   LineArgs a = line_args(g, p, uh, blines, hinv);
   a.cur = 3 * p.ntile;
-  a.top = top;
-  cudaMemsetAsync(top, 0, sizeof(unsigned long long), st);
+  a.range = range;
+  cudaMemsetAsync(range, 0, slice_range_bytes(p), st);
   const long long warps = (long long)p.Nu * a.cur * p.L;
-  k_slice_lines<WALK_MAX><<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(a);
-  WLG_LAUNCH_CHECK("slice_largest");
-}
-
-int slice_exponent(double top) {
-  for (int e = 0; e <= kSliceMaxExponent; e++)
-    if (top <= std::ldexp(1.98, e)) return e;
-  return -1;
+  k_slice_lines<WALK_RANGE><<<(unsigned)((warps + 3) / 4), 128, 0, st>>>(a);
+  WLG_LAUNCH_CHECK("slice_ranges");
 }
 
 void slice_lines(const Geo& g, const SlicePlan& p, const double* scale, int chunk,
@@ -861,8 +907,8 @@ void slice_finish(const Geo& g, const SlicePlan& p, const double* scale, int bc,
   const unsigned grid =
       (unsigned)std::min<size_t>((p.nwl + 255) / 256, (size_t)num_sms() * 16);
   const long long* s = reinterpret_cast<const long long*>(acc);
-  k_slice_finish<<<grid, 256, 0, st>>>(s, (long long)p.nwl, p.N0, p.mwlt, p.mwlr, p.L * p.L,
-                                       bc == 0, norm, scale, wl);
+  k_slice_finish<<<grid, 256, 0, st>>>(s, (long long)p.nwl, p.N0, p.mwlt, p.mwlr, p.L, bc == 0,
+                                       norm, scale, wl);
   WLG_LAUNCH_CHECK("slice_finish");
 }
 

@@ -208,23 +208,28 @@ struct SlicePlan {
 constexpr size_t kSliceBudget = (size_t)4 << 30;
 bool slice_plan(SlicePlan& p, const Geo& g, int bc, int msl, int mwlt, int mwlr,
                 size_t budget = kSliceBudget);
-// whether every line entry is known to stay within the digits' range, from max
-// |g g^dag - 1| and max |U^dag U - 1| over the levels (false for NaN)
-bool slice_in_range(double dev, double delta, int mwlr);
+// whether every line is known to stay within the digits' range and near enough to its
+// upper end, from max |g g^dag - 1| and max |U^dag U - 1| over the levels (false for
+// NaN); run, runs: columns and number of the FMA kernel's sums (slice_scales)
+bool slice_in_range(double dev, double delta, int mwlr, int run, int runs);
 // shared-memory limit and driver entry point (before any launch or capture)
 int slice_prepare(const SlicePlan& p);
 // *dev (device): max |U^dag U - 1| over the msl levels, as double bits
 void levels_deviation(const Geo& g, int msl, const double2* levels,
                       unsigned long long* dev, cudaStream_t st);
-// *top (device): the largest |entry| of all lines of all extents, as double bits
-void slice_largest(const Geo& g, const SlicePlan& p, const double* uh, const double* blines,
-                   const double* hinv, unsigned long long* top, cudaStream_t st);
-// the smallest e with top <= 1.98 2^e, -1 if it is above the largest allowed (the
-// classes left out grow as 2^(2e) against lines of norm 1)
+// range (device, slice_range_bytes): per extent and level the high word of the
+// largest entry's size, then [extent][level][B, A][slice] sums of squares in units
+// of 2^-30
+size_t slice_range_bytes(const SlicePlan& p);
+void slice_ranges(const Geo& g, const SlicePlan& p, const double* uh, const double* blines,
+                  const double* hinv, unsigned long long* range, cudaStream_t st);
+// the scales 2^-e [extent][level] from a range on the host; false where lines are
+// above 1.98 2^3, or so far apart in norm that the FMA kernel's sums are nearer
 constexpr int kSliceMaxExponent = 3;
-int slice_exponent(double top);
+bool slice_scales(const Geo& g, const SlicePlan& p, int run, int runs,
+                  const unsigned long long* range, double* scale);
 // digit planes of one chunk for R = 1..mwlr from the first lines, the recursion
-// links and H^-1, times *scale (device; a power of two, null: 1)
+// links and H^-1, times scale [extent][level] (device; powers of two, null: 1)
 void slice_lines(const Geo& g, const SlicePlan& p, const double* scale, int chunk,
                  const double* uh, const double* blines, const double* hinv, unsigned char* sa,
                  unsigned char* sb, cudaStream_t st);
