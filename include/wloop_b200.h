@@ -158,7 +158,7 @@ int wlg_batch_create(int nconf, const int* dims, const int* bcs, const wlg_wloop
                      int precision, int device, wlg_batch** out);
 int wlg_batch_destroy(wlg_batch* b);
 int wlg_batch_size(wlg_batch* b);
-/* device bytes held by the batch's field arena */
+/* device bytes held by the batch's field arena and its optional scratch */
 long long wlg_batch_bytes(wlg_batch* b);
 /* gauge field of configuration i from a host AoS su3_dble buffer */
 int wlg_batch_upload(wlg_batch* b, int i, const double* aos);
@@ -186,7 +186,8 @@ int wlg_batch_set_contract_shape(wlg_batch* b, int G, int SB, int nCB, int block
 /* on (default): the first run executes directly and captures the pipeline,
  * later runs replay the graph; off: every run executes directly */
 int wlg_batch_use_graph(wlg_batch* b, int on);
-/* device bytes a batch of these configurations would hold, or -1 */
+/* device bytes a batch of these configurations would hold, or -1; up to 4 x 512 MiB
+ * of it is scratch that a mixed batch of small lattices takes where it can be had */
 long long wlg_batch_estimate_bytes(int nconf, const int* dims, const int* bcs,
                                    const wlg_wloop_parms* parms, int precision);
 

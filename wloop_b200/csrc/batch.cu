@@ -130,6 +130,7 @@ struct wlg_batch {
   static constexpr int kSide = 4;
   cudaStream_t side[kSide] = {nullptr, nullptr, nullptr, nullptr};
   char* scratch[kSide] = {nullptr, nullptr, nullptr, nullptr};
+  size_t scratch_held = 0;
   cudaEvent_t fork = nullptr, join[kSide] = {nullptr, nullptr, nullptr, nullptr};
   float last_ms = 0.f;
   int kernels = 0;
@@ -860,6 +861,17 @@ void layout(wlg_batch* b) {
   b->staging_bytes = maxv * 4 * 144;
 }
 
+// bytes of scratch the lattices of stream k would run faster with (0: none)
+size_t scratch_bytes(const wlg_batch* b, int k) {
+  size_t most = 0;
+  for (size_t c = k; c < b->cfg.size(); c += wlg_batch::kSide) {
+    const PairPlan& q = b->cfg[c].pp_scratch;
+    if (q.npass > 0)
+      most = std::max(most, align256(q.bytes_a) + align256(q.bytes_b) + align256(q.bytes_p));
+  }
+  return most;
+}
+
 template <class P>
 int pool_alloc(wlg_batch* b, P** ptr, size_t bytes) {
   *ptr = nullptr;
@@ -971,10 +983,10 @@ int run_phase(wlg_batch* b, int phase) {
 
 }  // namespace
 
-extern "C" {
+namespace wlg {
 
-int wlg_batch_create(int nconf, const int* dims, const int* bcs, const wlg_wloop_parms* parms,
-                     int precision, int device, wlg_batch** out) {
+int batch_create(int nconf, const int* dims, const int* bcs, const wlg_wloop_parms* parms,
+                 int precision, int device, bool scratch, wlg_batch** out) {
   set_error("%s", "");
   if (nconf < 1 || !dims || !bcs || !parms || !out) {
     set_error("batch_create: bad arguments");
@@ -1042,14 +1054,10 @@ int wlg_batch_create(int nconf, const int* dims, const int* bcs, const wlg_wloop
     return -1;
   }
   // scratch of the lattice streams, where there is memory for it
-  for (int k = 0; k < wlg_batch::kSide; k++) {
-    size_t most = 0;
-    for (size_t c = k; c < b->cfg.size(); c += wlg_batch::kSide) {
-      const PairPlan& q = b->cfg[c].pp_scratch;
-      if (q.npass > 0)
-        most = std::max(most, align256(q.bytes_a) + align256(q.bytes_b) + align256(q.bytes_p));
-    }
+  for (int k = 0; scratch && k < wlg_batch::kSide; k++) {
+    const size_t most = scratch_bytes(b, k);
     if (most == 0 || pool_alloc(b, &b->scratch[k], most)) continue;
+    b->scratch_held += most;
     for (size_t c = k; c < b->cfg.size(); c += wlg_batch::kSide)
       b->cfg[c].pairs_scratch = b->cfg[c].pp_scratch.npass > 0;
   }
@@ -1062,6 +1070,38 @@ int wlg_batch_create(int nconf, const int* dims, const int* bcs, const wlg_wloop
   cudaEventCreate(&b->ev1);
   *out = b;
   return 0;
+}
+
+long long batch_need_bytes(int nconf, const int* dims, const int* bcs,
+                           const wlg_wloop_parms* parms, int precision, long long* scratch) {
+  if (nconf < 1 || !dims || !bcs || !parms) return -1;
+  if (precision != WLG_FP64 && precision != WLG_MIXED) return -1;
+  wlg_batch tmp;
+  tmp.prec = precision;
+  for (int c = 0; c < nconf; c++) {
+    Cfg f;
+    memset(&f, 0, sizeof(f));
+    if (check_lattice(dims + 4 * c, bcs[c])) return -1;
+    f.g = make_geo(dims + 4 * c);
+    f.bc = bcs[c];
+    f.p = parms[c];
+    if (check_parms(f.g, f.p)) return -1;
+    tmp.cfg.push_back(f);
+  }
+  layout(&tmp);
+  if (plan(&tmp)) return -1;
+  *scratch = 0;
+  for (int k = 0; k < wlg_batch::kSide; k++) *scratch += (long long)scratch_bytes(&tmp, k);
+  return (long long)(tmp.arena_bytes + tmp.pbuf_bytes + tmp.staging_bytes + (1 << 20));
+}
+
+}  // namespace wlg
+
+extern "C" {
+
+int wlg_batch_create(int nconf, const int* dims, const int* bcs, const wlg_wloop_parms* parms,
+                     int precision, int device, wlg_batch** out) {
+  return batch_create(nconf, dims, bcs, parms, precision, device, true, out);
 }
 
 int wlg_batch_destroy(wlg_batch* b) {
@@ -1123,7 +1163,9 @@ long long wlg_batch_pool_idle_bytes(int device) {
 
 int wlg_batch_size(wlg_batch* b) { return b ? (int)b->cfg.size() : 0; }
 
-long long wlg_batch_bytes(wlg_batch* b) { return b ? (long long)b->arena_bytes : 0; }
+long long wlg_batch_bytes(wlg_batch* b) {
+  return b ? (long long)(b->arena_bytes + b->scratch_held) : 0;
+}
 
 int wlg_batch_upload(wlg_batch* b, int i, const double* aos) {
   set_error("%s", "");
@@ -1257,26 +1299,13 @@ int wlg_batch_use_graph(wlg_batch* b, int on) {
   return 0;
 }
 
-// device bytes a batch of these configurations would hold (no allocation)
+// device bytes a batch of these configurations would hold, its optional scratch
+// included (no allocation)
 long long wlg_batch_estimate_bytes(int nconf, const int* dims, const int* bcs,
                                    const wlg_wloop_parms* parms, int precision) {
-  if (nconf < 1 || !dims || !bcs || !parms) return -1;
-  if (precision != WLG_FP64 && precision != WLG_MIXED) return -1;
-  wlg_batch tmp;
-  tmp.prec = precision;
-  for (int c = 0; c < nconf; c++) {
-    Cfg f;
-    memset(&f, 0, sizeof(f));
-    if (check_lattice(dims + 4 * c, bcs[c])) return -1;
-    f.g = make_geo(dims + 4 * c);
-    f.bc = bcs[c];
-    f.p = parms[c];
-    if (check_parms(f.g, f.p)) return -1;
-    tmp.cfg.push_back(f);
-  }
-  layout(&tmp);
-  if (plan(&tmp)) return -1;
-  return (long long)(tmp.arena_bytes + tmp.pbuf_bytes + tmp.staging_bytes + (1 << 20));
+  long long scratch = 0;
+  const long long need = batch_need_bytes(nconf, dims, bcs, parms, precision, &scratch);
+  return need < 0 ? need : need + scratch;
 }
 
 int wlg_batch_result(wlg_batch* b, int i, double* wl_mat) {

@@ -9,7 +9,8 @@
 // same precision (any lattices and loop parameters; up to max_batch), as long
 // as their device footprint fits both the server's memory budget (a fraction
 // of the HBM free at start, counting the batch pool's idle memory, minus what
-// the batches in flight reserve) and what cudaMemGetInfo reports free now.
+// the batches in flight reserve) and what cudaMemGetInfo reports free now.  A
+// batch's optional scratch is reserved, and taken, only where it fits as well.
 // A request at the head of the queue that does not fit yet does not block
 // the ones behind it: later requests that fit are admitted around it, until
 // the head has waited longer than the bypass limit; from then on nothing
@@ -35,6 +36,17 @@
 #include <vector>
 
 #include "../../include/wloop_b200.h"
+
+// batch.cu
+namespace wlg {
+// device bytes a batch of these configurations needs, and those of the scratch it
+// runs faster with
+long long batch_need_bytes(int nconf, const int* dims, const int* bcs,
+                           const wlg_wloop_parms* parms, int precision, long long* scratch);
+// wlg_batch_create, with or without that scratch
+int batch_create(int nconf, const int* dims, const int* bcs, const wlg_wloop_parms* parms,
+                 int precision, int device, bool scratch, wlg_batch** out);
+}  // namespace wlg
 
 namespace {
 
@@ -80,7 +92,8 @@ struct wlg_server {
 namespace {
 
 long long footprint(const wlg_request& r) {
-  return wlg_batch_estimate_bytes(1, r.n, &r.bc, &r.parms, r.precision);
+  long long scratch = 0;
+  return wlg::batch_need_bytes(1, r.n, &r.bc, &r.parms, r.precision, &scratch);
 }
 
 // requests that can share one batch: a batch has one precision
@@ -168,17 +181,6 @@ void worker(wlg_server* s) {
         if (!head_may_wait) break;  // a starving head starts alone
       }
     }
-    s->reserved += need;
-    double t0 = now_ms();
-    for (Req* q : group) {
-      q->state = 1;
-      q->t_start = t0;
-      q->batch_size = (int)group.size();
-    }
-    s->batches++;
-    lk.unlock();
-
-    // ---- one batch on this worker's stream ----
     const int k = (int)group.size();
     std::vector<int> dims(4 * k), bcs(k);
     std::vector<wlg_wloop_parms> parms(k);
@@ -191,10 +193,30 @@ void worker(wlg_server* s) {
       seeds[i] = group[i]->r.seed;
       eps[i] = group[i]->r.eps;
     }
+    // the batch's optional scratch, where the budget and the free memory hold it too
+    long long extra = 0;
+    wlg::batch_need_bytes(k, dims.data(), bcs.data(), parms.data(), group[0]->r.precision, &extra);
+    size_t fr = 0, tot = 0;
+    cudaMemGetInfo(&fr, &tot);
+    const bool scratch =
+        extra > 0 && s->reserved + need + extra <= s->budget &&
+        need + extra <= (long long)fr + wlg_batch_pool_idle_bytes(s->dev);
+    if (scratch) need += extra;
+    s->reserved += need;
+    double t0 = now_ms();
+    for (Req* q : group) {
+      q->state = 1;
+      q->t_start = t0;
+      q->batch_size = k;
+    }
+    s->batches++;
+    lk.unlock();
+
+    // ---- one batch on this worker's stream ----
     std::string err;
     wlg_batch* b = nullptr;
-    if (wlg_batch_create(k, dims.data(), bcs.data(), parms.data(), group[0]->r.precision, s->dev,
-                         &b)) {
+    if (wlg::batch_create(k, dims.data(), bcs.data(), parms.data(), group[0]->r.precision, s->dev,
+                          scratch, &b)) {
       err = wlg_last_error();
     } else {
       wlg_batch_use_graph(b, 0);  // each batch runs once
