@@ -1039,7 +1039,14 @@ int batch_create(int nconf, const int* dims, const int* bcs, const wlg_wloop_par
   }
   // the allocations are ordered on the batch's stream; complete them before
   // the host hands the buffers to copies on other streams
-  WLG_CUDA(cudaStreamSynchronize(b->st));
+  auto complete = [&]() {
+    const cudaError_t e = cudaStreamSynchronize(b->st);
+    if (e == cudaSuccess) return true;
+    set_error("batch_create: %s", cudaGetErrorString(e));
+    wlg_batch_destroy(b);
+    return false;
+  };
+  if (!complete()) return -1;
   for (int k = 0; k < wlg_batch::kSide; k++) {
     if (cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming) != cudaSuccess) {
@@ -1061,7 +1068,7 @@ int batch_create(int nconf, const int* dims, const int* bcs, const wlg_wloop_par
     for (size_t c = k; c < b->cfg.size(); c += wlg_batch::kSide)
       b->cfg[c].pairs_scratch = b->cfg[c].pp_scratch.npass > 0;
   }
-  WLG_CUDA(cudaStreamSynchronize(b->st));
+  if (!complete()) return -1;
   if (plan(b)) {
     wlg_batch_destroy(b);
     return -1;
