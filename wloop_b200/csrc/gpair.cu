@@ -148,7 +148,8 @@ __device__ __forceinline__ float4 lds4(unsigned addr) {
   float4 v;
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n"
                : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(addr));
+               : "r"(addr)
+               : "memory");
   return v;
 }
 
@@ -284,9 +285,11 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
           }
         }
-        // every lane's reads of the slot are done before lane 0 frees it (its
-        // arrive alone does not keep the last read of the other lanes ahead)
-        __threadfence_block();
+        // The slot's next content comes through the async proxy: each lane's reads
+        // are ordered before it by the lane's own proxy fence, then by the warp's
+        // barrier and lane 0's arrive (a release) and thread 0's wait (an acquire).
+        // Without any fence a warp freed slots before its last read.
+        fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(empty + s);
         if (++s == p.stages) {
