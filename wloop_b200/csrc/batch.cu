@@ -81,8 +81,6 @@ struct Op {
   int cfg, R;  // OP_GRAM_*: the lattice and the spatial extent
 };
 
-size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
-
 // most a lattice stream's scratch takes: a small lattice's level store would cut
 // its loop stage into passes too short to fill the GPU (16^3x32 with 4 levels:
 // 126 MB, 17 passes)
@@ -1146,6 +1144,7 @@ namespace wlg {
 void batch_pool_trim(int dev) {
   pool_trim(kBatchPool, dev);
   pool_trim(kCallPool, dev);
+  walk_trim(dev);
 }
 
 void* call_scratch(int dev, size_t bytes, cudaStream_t st) {
@@ -1165,7 +1164,7 @@ void call_scratch_trim(int dev) { pool_trim(kCallPool, dev); }
 extern "C" {
 
 long long wlg_batch_pool_idle_bytes(int device) {
-  return pool_idle(kBatchPool, device) + pool_idle(kCallPool, device);
+  return pool_idle(kBatchPool, device) + pool_idle(kCallPool, device) + walk_idle(device);
 }
 
 int wlg_batch_size(wlg_batch* b) { return b ? (int)b->cfg.size() : 0; }

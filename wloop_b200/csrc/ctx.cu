@@ -10,6 +10,7 @@
 #include <cmath>
 #include <atomic>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 #include <nvtx3/nvToolsExt.h>
@@ -57,6 +58,16 @@ struct DevBuf {
   cudaStream_t call = nullptr;  // from call_scratch: the stream to free it on
 };
 
+// idle buffers of walk_take, all devices, and the contexts that may want them
+struct WalkBuf {
+  int dev;
+  void* p;
+  size_t cap;
+};
+static std::mutex g_walk_mutex;
+static std::vector<WalkBuf> g_walk_idle;
+static std::map<int, int> g_contexts;  // live contexts per device
+
 struct ProfStat {
   double ms = 0.0;
   long long n = 0;
@@ -73,7 +84,7 @@ struct wlg_ctx {
   DevBuf gG, gH, gUh, gB, gA, gDev;
   // the lines of one chunk of columns, all extents (digit planes or FP32 level
   // pairs), the tensor-core product's integer sums, and its lines' range and scales
-  DevBuf gSa, gSb, gAcc, gRange;
+  DevBuf gS, gAcc, gRange;
   void* lines_at = nullptr;  // buffer holding the lines of length lines_len
   // after a temporal-gauge measurement the lines of length lines_lazy are
   // rebuilt from the level store when they are asked for
@@ -143,6 +154,99 @@ static int ensure_call(wlg_ctx* c, DevBuf& b, size_t bytes, size_t total, int ke
     }
   }
   return ensure(b, bytes);
+}
+
+static void* walk_reuse(int dev, size_t bytes, size_t* cap) {
+  std::lock_guard<std::mutex> lock(g_walk_mutex);
+  auto best = g_walk_idle.end();
+  for (auto it = g_walk_idle.begin(); it != g_walk_idle.end(); ++it)
+    if (it->dev == dev && it->cap >= bytes && (best == g_walk_idle.end() || it->cap < best->cap))
+      best = it;
+  if (best == g_walk_idle.end()) return nullptr;
+  void* p = best->p;
+  *cap = best->cap;
+  g_walk_idle.erase(best);
+  return p;
+}
+
+namespace wlg {
+void* walk_take(int dev, size_t bytes, size_t* cap) {
+  if (void* p = walk_reuse(dev, bytes, cap)) return p;
+  void* p = nullptr;
+  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    batch_pool_trim(dev);
+    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+  }
+  *cap = bytes;
+  return p;
+}
+
+void walk_give(int dev, void* p, size_t cap) {
+  std::vector<void*> drop;
+  {
+    std::lock_guard<std::mutex> lock(g_walk_mutex);
+    g_walk_idle.push_back({dev, p, cap});
+    // the largest stay: they serve smaller lattices too
+    for (;;) {
+      size_t idle = 0;
+      auto least = g_walk_idle.end();
+      for (auto it = g_walk_idle.begin(); it != g_walk_idle.end(); ++it) {
+        if (it->dev != dev) continue;
+        idle += it->cap;
+        if (least == g_walk_idle.end() || it->cap < least->cap) least = it;
+      }
+      if (idle <= kWalkScratch) break;
+      drop.push_back(least->p);
+      g_walk_idle.erase(least);
+    }
+  }
+  for (void* q : drop) cudaFree(q);
+}
+
+void walk_trim(int dev) {
+  std::vector<void*> drop;
+  {
+    std::lock_guard<std::mutex> lock(g_walk_mutex);
+    for (size_t i = 0; i < g_walk_idle.size();)
+      if (g_walk_idle[i].dev == dev) {
+        drop.push_back(g_walk_idle[i].p);
+        g_walk_idle.erase(g_walk_idle.begin() + i);
+      } else {
+        i++;
+      }
+  }
+  for (void* p : drop) cudaFree(p);
+}
+
+long long walk_idle(int dev) {
+  std::lock_guard<std::mutex> lock(g_walk_mutex);
+  long long idle = 0;
+  for (const WalkBuf& w : g_walk_idle) idle += w.dev == dev ? (long long)w.cap : 0;
+  return idle;
+}
+}  // namespace wlg
+
+// The lines of a chunk, A then B.  The loop stage gives them back when its stream
+// has been waited for, so that any other context can have them.
+static void give_walk(wlg_ctx* c) {
+  if (c->gS.p) {
+    cudaStreamSynchronize(c->st);
+    walk_give(c->dev, c->gS.p, c->gS.cap);
+  }
+  c->gS = DevBuf();
+}
+
+static int ensure_walk(wlg_ctx* c, size_t bytes_a, size_t bytes_b) {
+  give_walk(c);
+  const size_t bytes = align256(bytes_a) + bytes_b;
+  c->gS.p = walk_take(c->dev, bytes, &c->gS.cap);
+  if (c->gS.p) return 0;
+  set_error("cudaMalloc(%zu bytes) failed", bytes);
+  return -1;
 }
 
 // bytes of one direction array (tiled layout, common.cuh) and of ndir of them
@@ -417,8 +521,8 @@ static void release_idle_scratch(wlg_ctx* c) {
   release(c->apeB);
   release(c->dl);
   release(c->staging);
-  release(c->gSa);
-  release(c->gSb);
+  give_walk(c);
+  walk_trim(c->dev);
   set_error("%s", "");
 }
 
@@ -433,8 +537,8 @@ static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan&
   const size_t nb = gp.A * sizeof(double) * 3 * msl;
   const size_t range_bytes = slice_range_bytes(sp);
   auto alloc = [&]() {
-    return ensure(c->gUh, nb) || ensure(c->gB, nb) || ensure(c->gSa, sp.bytes_a) ||
-           ensure(c->gSb, sp.bytes_b) || ensure(c->gAcc, sp.acc_bytes) ||
+    return ensure(c->gUh, nb) || ensure(c->gB, nb) ||
+           ensure_walk(c, sp.bytes_a, sp.bytes_b) || ensure(c->gAcc, sp.acc_bytes) ||
            (!in_range && ensure(c->gRange, range_bytes + sizeof(double) * p->mwlr * msl)) ||
            ensure(c->wl, sizeof(double) * sp.nwl);
   };
@@ -442,14 +546,15 @@ static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan&
     release_idle_scratch(c);
     if (alloc()) {
       set_error("%s", "");
-      release(c->gSa);
-      release(c->gSb);
+      give_walk(c);
       return 1;
     }
   }
   double* uh = (double*)c->gUh.p;
   double* bl = (double*)c->gB.p;
   const double* hinv = (const double*)c->gH.p;
+  unsigned char* sa = (unsigned char*)c->gS.p;
+  unsigned char* sb = sa + align256(sp.bytes_a);
   unsigned long long* acc = (unsigned long long*)c->gAcc.p;
   int* fail = (int*)((unsigned long long*)c->gDev.p + 2);
   WLG_CUDA(cudaMemsetAsync(acc, 0, sp.acc_bytes, c->st));
@@ -468,7 +573,10 @@ static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan&
     std::vector<double> scales((size_t)p->mwlr * msl);
     WLG_CUDA(cudaMemcpyAsync(seen.data(), range, range_bytes, cudaMemcpyDeviceToHost, c->st));
     WLG_CUDA(cudaStreamSynchronize(c->st));
-    if (!slice_scales(g, sp, gp.cpc * 32, gp.nsplit, seen.data(), scales.data())) return 1;
+    if (!slice_scales(g, sp, gp.cpc * 32, gp.nsplit, seen.data(), scales.data())) {
+      give_walk(c);
+      return 1;
+    }
     double* at = (double*)((char*)range + range_bytes);
     WLG_CUDA(cudaMemcpyAsync(at, scales.data(), scales.size() * sizeof(double),
                              cudaMemcpyHostToDevice, c->st));
@@ -482,12 +590,11 @@ static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan&
   for (int ch = 0; ch < sp.nchunk; ch++) {
     {
       ProfScope ps(c, "lines");
-      slice_lines(g, sp, scale, ch, uh, bl, hinv, (unsigned char*)c->gSa.p,
-                  (unsigned char*)c->gSb.p, c->st);
+      slice_lines(g, sp, scale, ch, uh, bl, hinv, sa, sb, c->st);
     }
     {
       ProfScope ps(c, "contract");
-      slice_gram(sp, ch, (unsigned char*)c->gSa.p, (unsigned char*)c->gSb.p, acc, fail, c->st);
+      slice_gram(sp, ch, sa, sb, acc, fail, c->st);
     }
   }
   {
@@ -501,6 +608,7 @@ static int do_loops_slices(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan&
     WLG_CUDA(cudaMemcpyAsync(wl_mat, c->wl.p, sizeof(double) * sp.nwl, cudaMemcpyDeviceToHost,
                              c->st));
   WLG_CUDA(cudaStreamSynchronize(c->st));
+  give_walk(c);
   if (failed) {
     set_error("wloop_sum: the Gram product's operand copies did not arrive in time");
     return -1;
@@ -519,16 +627,15 @@ static int do_loops_pairs(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan& 
   const size_t nb = gp.A * sizeof(float) * 3 * msl;
   const size_t nwl = (size_t)msl * msl * p->mwlt * p->mwlr * g.n[0];
   auto alloc = [&]() {
-    return ensure(c->gUh, nb) || ensure(c->gB, nb) || ensure(c->gSa, pp.bytes_a) ||
-           ensure(c->gSb, pp.bytes_b) || ensure(c->partial, pp.bytes_p) ||
+    return ensure(c->gUh, nb) || ensure(c->gB, nb) ||
+           ensure_walk(c, pp.bytes_a, pp.bytes_b) || ensure(c->partial, pp.bytes_p) ||
            ensure(c->wl, sizeof(double) * nwl);
   };
   if (alloc()) {
     release_idle_scratch(c);
     if (alloc()) {
       set_error("%s", "");
-      release(c->gSa);
-      release(c->gSb);
+      give_walk(c);
       return 1;
     }
   }
@@ -539,6 +646,8 @@ static int do_loops_pairs(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan& 
   float* uh = (float*)c->gUh.p;
   float* bl = (float*)c->gB.p;
   const double* hinv = (const double*)c->gH.p;
+  char* pa = (char*)c->gS.p;
+  char* pb = pa + align256(pp.bytes_a);
   float* hf = (float*)c->gG.p;  // H^-1 in FP32 takes the place of g, dead by then
   int* fail = (int*)((unsigned long long*)c->gDev.p + 2);
   WLG_CUDA(cudaMemsetAsync(fail, 0, sizeof(int), c->st));
@@ -551,11 +660,11 @@ static int do_loops_pairs(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan& 
   for (int k = 0; k < pp.npass; k++) {
     {
       ProfScope ps(c, "lines");
-      pair_lines(g, pp, k, uh, bl, hf, c->gSa.p, c->gSb.p, c->st);
+      pair_lines(g, pp, k, uh, bl, hf, pa, pb, c->st);
     }
     {
       ProfScope ps(c, "contract");
-      pair_gram(pp, k, c->gSa.p, c->gSb.p, (float*)c->partial.p, fail, c->st);
+      pair_gram(pp, k, pa, pb, (float*)c->partial.p, fail, c->st);
     }
     {
       ProfScope ps(c, "reduce");
@@ -568,6 +677,7 @@ static int do_loops_pairs(wlg_ctx* c, const wlg_wloop_parms* p, const GramPlan& 
   if (wl_mat)
     WLG_CUDA(cudaMemcpyAsync(wl_mat, c->wl.p, sizeof(double) * nwl, cudaMemcpyDeviceToHost, c->st));
   WLG_CUDA(cudaStreamSynchronize(c->st));
+  give_walk(c);
   if (failed) {
     set_error("wloop_sum: the Gram product's operand copies did not arrive in time");
     return -1;
@@ -836,6 +946,10 @@ int wlg_create(const int n[4], int bc, int precision, int device, wlg_ctx** out)
     return -1;
   }
   WLG_CUDA(cudaMemsetAsync(c->U.p, 0, field_bytes(c, 4), c->st));
+  {
+    std::lock_guard<std::mutex> lock(g_walk_mutex);
+    g_contexts[device]++;
+  }
   *out = c;
   return 0;
 }
@@ -859,8 +973,7 @@ int wlg_free_scratch(wlg_ctx* c) {
   release(c->gB);
   release(c->gA);
   release(c->gDev);
-  release(c->gSa);
-  release(c->gSb);
+  give_walk(c);
   release(c->gAcc);
   release(c->gRange);
   c->lines_at = nullptr;
@@ -869,6 +982,7 @@ int wlg_free_scratch(wlg_ctx* c) {
   release(c->partial);
   release(c->staging);
   call_scratch_trim(c->dev);
+  walk_trim(c->dev);
   return 0;
 }
 
@@ -879,8 +993,9 @@ int wlg_destroy(wlg_ctx* c) {
   if (c->cst) cudaStreamSynchronize(c->cst);
   harvest(c);
   DevBuf* all[] = {&c->U, &c->U0, &c->bar, &c->til, &c->apeA, &c->apeB, &c->dl, &c->levels, &c->lines, &c->lines2,
-                   &c->gG, &c->gH, &c->gUh, &c->gB, &c->gA, &c->gDev, &c->gSa, &c->gSb, &c->gAcc, &c->gRange, &c->partial, &c->wl, &c->plaq_part, &c->plaq_out, &c->plaq_count, &c->staging, &c->ipt,
+                   &c->gG, &c->gH, &c->gUh, &c->gB, &c->gA, &c->gDev, &c->gAcc, &c->gRange, &c->partial, &c->wl, &c->plaq_part, &c->plaq_out, &c->plaq_count, &c->staging, &c->ipt,
                    &c->prefetch_buf};
+  give_walk(c);
   for (DevBuf* b : all) release(*b);
   for (cudaEvent_t e : c->evpool) cudaEventDestroy(e);
   if (c->cst) {
@@ -890,6 +1005,12 @@ int wlg_destroy(wlg_ctx* c) {
   }
   cudaStreamDestroy(c->st);
   call_scratch_trim(c->dev);
+  bool last;
+  {
+    std::lock_guard<std::mutex> lock(g_walk_mutex);
+    last = --g_contexts[c->dev] == 0;
+  }
+  if (last) walk_trim(c->dev);
   delete c;
   return 0;
 }

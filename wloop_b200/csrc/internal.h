@@ -290,6 +290,8 @@ RArgs reduce_args(const Geo& g, const ContractPlan& p, int msl, int mwlt, int mw
 void contract_reduce_batch(const RArgs* A, const long long* pre, int n, long long total,
                            cudaStream_t st);
 
+inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
+
 // ---- memory pools (batch.cu) -------------------------------------------------
 // gives the idle memory the pools of device dev keep back to the device
 void batch_pool_trim(int dev);
@@ -300,6 +302,17 @@ void batch_pool_trim(int dev);
 constexpr size_t kCallScratch = (size_t)1 << 30;
 void* call_scratch(int dev, size_t bytes, cudaStream_t st);
 void call_scratch_trim(int dev);
+// Buffers for the lines of a chunk (kSliceBudget, kPairBudget: up to 4 GiB), which a
+// context needs while its loop stage runs: kept by every context, they took a
+// 32 x 16^3 mixed one from 0.9 GB to 2.9.  The device keeps at most kWalkScratch of
+// them idle, what two contexts that measure at a time use.  They come from cudaMalloc,
+// not from a pool of the runtime's: 4 GiB take 4 ms (25 from a pool).  walk_give: no
+// work of the caller uses the buffer any more.  (ctx.cu)
+constexpr size_t kWalkScratch = (size_t)9 << 30;
+void* walk_take(int dev, size_t bytes, size_t* cap);
+void walk_give(int dev, void* p, size_t cap);
+void walk_trim(int dev);
+long long walk_idle(int dev);
 
 // ---- layout (layout.cu) ---------------------------------------------------
 // AoS lexicographic FP64 [V][4][18] <-> SoA field of type T (directions [mu0,mu1)).
