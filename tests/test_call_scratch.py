@@ -63,3 +63,27 @@ def test_pool_is_bounded_and_given_back():
         b.free_scratch()
         assert lib.wlg_batch_pool_idle_bytes(0) <= before
         assert torch.cuda.mem_get_info(0)[0] >= free + idle
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("call", [lambda c: c.hyp_links(0.75, 0.6, 0.3),
+                                  lambda c: c.ape_links(0.1, nsweeps=3),
+                                  lambda c: c.hyp_spatial_links(0.75, 0.6)],
+                         ids=["hyp", "ape", "hyp_spatial"])
+def test_scratch_comes_from_the_pool_and_returns_at_once(call):
+    """The pool of the calls alone (other pools' idle memory stays what it was), and
+    another context gives its memory back right after the call."""
+    import torch
+    n = (32, 16, 16, 20)
+    with Context(n, 3, "fp64") as c, Context((4, 4, 4, 4), 3) as other:
+        c.generate(3, 0.3)
+        c.sync()
+        other.free_scratch()
+        before = lib.wlg_batch_pool_idle_bytes(0)
+        free = torch.cuda.mem_get_info(0)[0]
+        call(c)
+        idle = lib.wlg_batch_pool_idle_bytes(0) - before
+        assert 4 * 163840 * 144 <= idle <= LIMIT  # at least four directions
+        other.free_scratch()
+        assert lib.wlg_batch_pool_idle_bytes(0) <= before
+        assert torch.cuda.mem_get_info(0)[0] >= free - (2 << 20)

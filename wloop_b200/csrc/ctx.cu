@@ -8,6 +8,7 @@
 #include <string.h>
 #include <algorithm>
 #include <cmath>
+#include <initializer_list>
 #include <atomic>
 #include <map>
 #include <mutex>
@@ -154,6 +155,16 @@ static int ensure_call(wlg_ctx* c, DevBuf& b, size_t bytes, size_t total, int ke
     }
   }
   return ensure(b, bytes);
+}
+
+// the end of a call without `keep`: its scratch is given back
+static int end_call(wlg_ctx* c, std::initializer_list<DevBuf*> bufs) {
+  for (DevBuf* b : bufs)
+    if (b->call) release(*b);
+  // the pool can return to the device only what the host has seen freed
+  WLG_CUDA(cudaStreamSynchronize(c->st));
+  for (DevBuf* b : bufs) release(*b);
+  return 0;
 }
 
 static void* walk_reuse(int dev, size_t bytes, size_t* cap) {
@@ -360,11 +371,7 @@ template <class T> static int do_hyp(wlg_ctx* c, double a1, double a2, double a3
     hyp_level1<T>(c->g, U, (const typename V2<T>::t*)c->til.p, a1, proj, piter, mu0, mu1, c->bc,
                   c->st);
   }
-  if (!keep) {
-    WLG_CUDA(cudaStreamSynchronize(c->st));
-    release(c->bar);
-    release(c->til);
-  }
+  if (!keep && end_call(c, {&c->bar, &c->til})) return -1;
   return finish("hyp");
 }
 
@@ -389,10 +396,7 @@ template <class T> static int do_ape(wlg_ctx* c, double alpha, int proj, int pit
     WLG_CUDA(cudaMemcpyAsync((char*)c->U.p + off, (char*)c->apeA.p + off,
                              field_bytes(c, 4 - mu0), cudaMemcpyDeviceToDevice, c->st));
   }
-  if (!keep) {
-    WLG_CUDA(cudaStreamSynchronize(c->st));
-    release(c->apeA);
-  }
+  if (!keep && end_call(c, {&c->apeA})) return -1;
   return finish("ape");
 }
 
@@ -416,10 +420,7 @@ template <class T> static int do_hyp_spatial(wlg_ctx* c, double a1, double a2, i
     for (int i = 0; i < nsweeps; i++)
       if (hyp3_sweep<T>(c, U, U, a1, a2, proj, piter)) return -1;
   }
-  if (!keep) {
-    WLG_CUDA(cudaStreamSynchronize(c->st));
-    release(c->dl);
-  }
+  if (!keep && end_call(c, {&c->dl})) return -1;
   return finish("hyp_spatial");
 }
 
