@@ -702,14 +702,16 @@ static int do_loops_gram(wlg_ctx* c, const wlg_wloop_parms* p, double* wl_mat) {
   // the form needs projected smearing (the projection keeps the temporal
   // links near SU(3), so g stays well conditioned)
   if (p->proj_iter < 3) return 1;
-  const bool fma_ok = gram_plan(gp, g, c->bc, msl, p->mwlt, fp64, &c->gtune);
-  if (!fma_ok) return 1;
+  // (the digit product needs no plan of the FMA kernel, but what it declines does)
+  if (!gram_plan(gp, g, c->bc, msl, p->mwlt, fp64, &c->gtune)) return 1;
   // a tuned shape asks for the FMA kernel
-  bool slices = fp64 && !c->gtune.set() && slice_plan(sp, g, c->bc, msl, p->mwlt, p->mwlr) &&
-                slice_prepare(sp) == 0;
+  const bool walk = !c->gtune.set();
   PairPlan pp;
-  const bool pairs = !fp64 && !c->gtune.set() &&
-                     pair_plan(pp, gp, g, msl, p->mwlt, p->mwlr) && pair_prepare(pp) == 0;
+  const bool slices = walk && fp64 && slice_plan(sp, g, c->bc, msl, p->mwlt, p->mwlr) &&
+                      slice_prepare(sp) == 0;
+  const bool pairs = walk && !fp64 && pair_plan(pp, gp, g, msl, p->mwlt, p->mwlr) &&
+                     pair_prepare(pp) == 0;
+  set_error("%s", "");  // one that cannot be prepared leaves the measurement to the FMA kernel
   if (gram_prepare(gp)) return -1;
   const size_t nb = gp.A * sizeof(T) * 3 * msl, na = gp.Aa * sizeof(T) * 3 * msl;
   const size_t nwl = (size_t)msl * msl * p->mwlt * p->mwlr * g.n[0];
