@@ -542,13 +542,17 @@ def run_ours(args, rank, world, local):
         achieved *= 28
         peak = 4500.0
         peak_src = "nominal dense int8 rate (no measured one)"
-    traffic = load_traffic().get(args.precision + ("_gram" if form == 11 else ""))
+    measured = {}
     peaks_file = os.path.join(ROOT, "MEASURED_PEAKS.json")
-    hbm, hbm_src = None, None
     if os.path.exists(peaks_file):
         with open(peaks_file) as f:
-            hbm = json.load(f).get("hbm_gbs")
-        hbm_src = "MEASURED_PEAKS.json hbm_gbs (of measured)"
+            measured = json.load(f)
+    if digits and measured.get("bf16_tflops_sustained"):
+        peak = 2.0 * measured["bf16_tflops_sustained"]
+        peak_src = ("twice the sustained cuBLAS bf16 rate (of measured): int8 products run at "
+                    "twice the bf16 rate")
+    traffic = load_traffic().get(args.precision + ("_gram" if form == 11 else ""))
+    hbm, hbm_src = measured.get("hbm_gbs"), "MEASURED_PEAKS.json hbm_gbs (of measured)"
     if not hbm:
         # an earlier STREAM-style copy measurement on B200s of this kind
         hbm, hbm_src = HBM_FALLBACK_GBS, "6650 GB/s earlier B200 copy measurement (of fallback)"
