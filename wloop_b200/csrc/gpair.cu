@@ -112,8 +112,8 @@ __global__ void __launch_bounds__(128, 4) k_pair_lines(PairLineArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// The Gram product.  An item is (R, run, start-slice block); one CTA per SM
-// walks items.  Thread 0 stages 16 columns at a time, stages - 2 ahead: one TMA
+// The Gram product.  An item is (R, run, start-slice block); a CTA walks items,
+// one CTA per SM (up to four where blocks are small).  Thread 0 stages 16 columns at a time, stages - 2 ahead: one TMA
 // box of the block's BXp start slices and one of its NYBp partner slices, all
 // level pairs, as 128-byte rows (128-byte swizzle; slice counts padded to 8, so
 // a thread's swizzle is fixed).  Thread (i, gq) owns start slice

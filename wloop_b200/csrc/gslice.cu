@@ -15,16 +15,20 @@
 // finds the largest entry and the least norm of a slice per extent and level, and
 // the lines of each extent and level are scaled by 2^-e for the smallest e <= 3
 // that holds them, unless their norm is so far below it that FP64 FMAs would be
-// nearer (slice_scales).  The FMA kernel of gram.cu measures the rest, and a NaN
-// anywhere fails every comparison.  A dot product is then
+// nearer (slice_scales; 32 x 20^3, msl 4, three levels of spatial HYP: 10.4 ms a
+// measurement with the walk and the digits, 12.3 with the FMA kernel).  The FMA kernel of
+// gram.cu measures the rest, and a NaN anywhere fails every comparison.  A dot
+// product is then
 //     sum_c a_c b_c = sum_m 2^(-12-8m) C_m,   C_m = sum_{i+j=m} q_a,i . q_b,j
 // over the classes m < 7.  The classes that are left out and the rounding of x
-// are unbiased digits of size 2^-54 per column, and shrink against the sum
-// with the square root of the 54 N1 N2 N3 columns, to below 1e-17 of W; the
-// integer sums are exact, so a result does not depend on how columns are split
-// over blocks or in which order blocks add theirs.  Against 64-bit loops of
-// the same fields W is 1.3e-16 .. 4.9e-16 off (2-norm) where the FMA kernel's
-// FP64 sums are 4.1e-16 .. 6.5e-16 off.
+// are absolute errors of 4.5e-17 a column (of lines scaled to the digits' range) that
+// add up as random ones: of W, a mean over 9 N1 N2 N3, about 3.7e-17 / sqrt(N1 N2 N3)
+// times the lines' 2^(e1 + e2), whatever W is (emulated: 4.5e-18 at 4^3, 3.8e-19 at 20^3).
+// The integer sums are exact, so a result does not depend on how columns are
+// split over blocks or in which order blocks add theirs.  FP64 FMAs of the same
+// lines are 2.4e-18 .. 2.4e-17 off where W is small, more where it is not.  Against
+// 64-bit loops of the same fields W is 1.3e-16 .. 4.9e-16 off (2-norm, lines included)
+// where the FMA kernel's sums are 4.1e-16 .. 6.5e-16 off.
 //
 // The mixed form keeps FP32 FMAs (gpair.cu): its sums' rounding is part of its
 // results.

@@ -1,4 +1,4 @@
-// mbar.cuh -- mbarriers, bounded waits and bulk copies (loops.cu, gslice.cu)
+// mbar.cuh -- mbarriers, bounded waits and bulk copies (loops.cu, gslice.cu, gpair.cu)
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

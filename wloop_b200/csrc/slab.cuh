@@ -1,4 +1,4 @@
-// slab.cuh -- the temporal-gauge slab layout (gram.cu, gslice.cu): component c
+// slab.cuh -- the temporal-gauge slab layout (gram.cu, gslice.cu, gpair.cu): component c
 // (= 2 e + {0: re, 1: im} of entry e, row-major) of site (y0, j) of one array
 // at ((y0 * ntile + j / 32) * 18 + c) * 32 + j % 32, ntile = ceil(vs / 32).
 #pragma once
