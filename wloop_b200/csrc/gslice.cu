@@ -16,7 +16,7 @@
 // the lines of each extent and level are scaled by 2^-e for the smallest e <= 3
 // that holds them, unless their norm is so far below it that FP64 FMAs would be
 // nearer (slice_scales; 32 x 20^3, msl 4, three levels of spatial HYP: 10.4 ms a
-// measurement with the walk and the digits, 12.3 with the FMA kernel).  The FMA kernel of
+// measurement with the walk and the digits, 11.8 with the FMA kernel).  The FMA kernel of
 // gram.cu measures the rest, and a NaN anywhere fails every comparison.  A dot
 // product is then
 //     sum_c a_c b_c = sum_m 2^(-12-8m) C_m,   C_m = sum_{i+j=m} q_a,i . q_b,j
